@@ -1100,51 +1100,81 @@ int hexa_oc_update(hexa_ctx* h, int64_t n, const double* x, const double* dc, co
   const double* vd = stage_in<double>(c, dv, n, "o_dv");
   double* od = out_buf<double>(c, x_out, n, "o_out");
   double* lam_d = c.vec<double>("o_lam", 32);
+  double* t = c.vec<double>("o_t", n);
+  double* lo_d = c.vec<double>("o_lo", n);
+  double* hi_d = c.vec<double>("o_hi", n);
+  OcState* os = c.vec<OcState>("o_state", 1);
   const int nb = (int)std::min<long long>((n + 255) / 256, 152 * 4);
-  if (!xd || !cd || !vd || !od || !lam_d || !c.ensure_partials((size_t)nb * 32 + 64)) return HEXA_ERR_NOMEM;
-  std::vector<double> part((size_t)nb * 32);
-  // Bisection of the 88-line code on lambda in [0, 1e9] until
-  // (l2-l1)/(l1+l2) <= 1e-3 is replaced by the same sequence of midpoints to a
-  // tighter 1e-12, evaluated five levels of the bisection tree (31 multipliers)
-  // per pass over the elements.
+  if (!xd || !cd || !vd || !od || !lam_d || !t || !lo_d || !hi_d || !os || !c.ensure_partials((size_t)nb * 32 + 64))
+    return HEXA_ERR_NOMEM;
+  // The multiplier is that of the 88-line code's bisection on lambda in
+  // [0, 1e9], carried to (l2 - l1)/(l1 + l2) <= 1e-12 where that stops at
+  // 1e-3.  The volume does not rise with lambda, so every comparison of the
+  // bisection follows from the root of V(lambda) = target: the device finds
+  // the root (FP32 bracket, then Newton steps on the FP64 volume, about five
+  // passes over the elements), and the midpoints are walked here.
   double l1 = 0.0, l2 = 1e9, last_mid = 0.5 * (l1 + l2);
   const double target = volfrac * (double)n;
-  int passes = 0;
   cudaEventRecord(c.ev[0], c.st);
-  while ((l2 - l1) / (l1 + l2) > 1e-12 && passes < 64) {
-    double lams[31];
-    // heap order: node t has children 2t+1, 2t+2 (left = [l1,mid], right = [mid,l2])
-    double lo[31], hi[31];
-    lo[0] = l1;
-    hi[0] = l2;
-    for (int t = 0; t < 31; ++t) {
-      lams[t] = 0.5 * (hi[t] + lo[t]);
-      if (2 * t + 2 < 31) {
-        lo[2 * t + 1] = lo[t];
-        hi[2 * t + 1] = lams[t];
-        lo[2 * t + 2] = lams[t];
-        hi[2 * t + 2] = hi[t];
-      }
+  cudaMemsetAsync(os, 0, sizeof(OcState), c.st);
+  launch_oc_prepare(xd, cd, vd, n, move, target, t, lo_d, hi_d, c.partials, os, nb, c.st);
+  c.launches++;
+  OcState* hos = reinterpret_cast<OcState*>(c.hscal + 32);
+  static_assert(sizeof(OcState) <= 16 * sizeof(double), "OcState exceeds its host landing slots");
+  hos->state = 0;
+  for (int round = 0; round < 8 && hos->state == 0; ++round) {
+    for (int k = 0; k < 6; ++k) launch_oc_step(t, lo_d, hi_d, n, target, c.partials, os, nb, c.st);
+    c.launches += 6;
+    cudaMemcpyAsync(hos, os, sizeof(OcState), cudaMemcpyDeviceToHost, c.st);
+    if (cudaStreamSynchronize(c.st) != cudaSuccess) return set_err(h, HEXA_ERR_CUDA, "oc search failed");
+  }
+  if (hos->state == 1) {
+    const double lam_root = 1.0 / (hos->root * hos->root);
+    for (int level = 0; level < 320 && (l2 - l1) / (l1 + l2) > 1e-12; ++level) {
+      last_mid = 0.5 * (l1 + l2);
+      if (last_mid < lam_root) l1 = last_mid;  // V(mid) > target
+      else l2 = last_mid;
     }
-    cudaMemcpyAsync(lam_d, lams, sizeof(lams), cudaMemcpyHostToDevice, c.st);
-    launch_oc_volumes(xd, cd, vd, n, lam_d, 31, move, c.partials, nb, c.st);
-    c.launches++;
-    cudaMemcpyAsync(part.data(), c.partials, (size_t)nb * 32 * sizeof(double), cudaMemcpyDeviceToHost, c.st);
-    if (cudaStreamSynchronize(c.st) != cudaSuccess) return set_err(h, HEXA_ERR_CUDA, "oc pass failed");
-    ++passes;
-    int t = 0;
-    for (int depth = 0; depth < 5; ++depth) {
-      if (!((l2 - l1) / (l1 + l2) > 1e-12)) break;
-      double vol = 0.0;
-      for (int b = 0; b < nb; ++b) vol += part[(size_t)b * 32 + t];
-      const double lmid = lams[t];
-      last_mid = lmid;
-      if (vol > target) {
-        l1 = lmid;
-        t = 2 * t + 2;
-      } else {
-        l2 = lmid;
-        t = 2 * t + 1;
+  } else {
+    // no root in the search's range: every comparison evaluated, five levels of
+    // the bisection tree (31 multipliers) per pass over the elements
+    std::vector<double> part((size_t)nb * 32);
+    int passes = 0;
+    while ((l2 - l1) / (l1 + l2) > 1e-12 && passes < 64) {
+      double lams[31];
+      // heap order: node q has children 2q+1, 2q+2 (left = [l1,mid], right = [mid,l2])
+      double lo[31], hi[31];
+      lo[0] = l1;
+      hi[0] = l2;
+      for (int q = 0; q < 31; ++q) {
+        lams[q] = 0.5 * (hi[q] + lo[q]);
+        if (2 * q + 2 < 31) {
+          lo[2 * q + 1] = lo[q];
+          hi[2 * q + 1] = lams[q];
+          lo[2 * q + 2] = lams[q];
+          hi[2 * q + 2] = hi[q];
+        }
+      }
+      cudaMemcpyAsync(lam_d, lams, sizeof(lams), cudaMemcpyHostToDevice, c.st);
+      launch_oc_volumes(t, lo_d, hi_d, n, lam_d, 31, c.partials, nb, c.st);
+      c.launches++;
+      cudaMemcpyAsync(part.data(), c.partials, (size_t)nb * 32 * sizeof(double), cudaMemcpyDeviceToHost, c.st);
+      if (cudaStreamSynchronize(c.st) != cudaSuccess) return set_err(h, HEXA_ERR_CUDA, "oc pass failed");
+      ++passes;
+      int q = 0;
+      for (int depth = 0; depth < 5; ++depth) {
+        if (!((l2 - l1) / (l1 + l2) > 1e-12)) break;
+        double vol = 0.0;
+        for (int b = 0; b < nb; ++b) vol += part[(size_t)b * 32 + q];
+        const double lmid = lams[q];
+        last_mid = lmid;
+        if (vol > target) {
+          l1 = lmid;
+          q = 2 * q + 2;
+        } else {
+          l2 = lmid;
+          q = 2 * q + 1;
+        }
       }
     }
   }

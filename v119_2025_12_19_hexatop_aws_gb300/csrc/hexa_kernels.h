@@ -153,9 +153,19 @@ void launch_simp_factors(const double* rho, double Emin, double E0, double penal
 void launch_sensitivities(const Grid& g, const ModalK<double>& K, const double* rho,
                           const double* u, double Emin, double E0, double penal, double* dc,
                           const RedArgs& red, cudaStream_t st);
-void launch_oc_volumes(const double* x, const double* dc, const double* dv, long long n,
-                       const double* lam, int nlam, double move, double* partials, int nblocks,
-                       cudaStream_t st);
+// Search for the multiplier of the OC update (topo.cu): state 0 running, 1
+// root found, 2 no root in the range.
+struct OcState {
+  double s, s_lo, s_hi, root;
+  int state;
+  unsigned ticket;
+};
+void launch_oc_prepare(const double* x, const double* dc, const double* dv, long long n, double move, double target,
+                       double* t, double* lo, double* hi, double* part, OcState* st, int nblocks, cudaStream_t s);
+void launch_oc_step(const double* t, const double* lo, const double* hi, long long n, double target, double* part,
+                    OcState* st, int nblocks, cudaStream_t s);
+void launch_oc_volumes(const double* t, const double* lo, const double* hi, long long n, const double* lam, int nlam,
+                       double* partials, int nblocks, cudaStream_t st);
 void launch_oc_apply(const double* x, const double* dc, const double* dv, long long n, double lam,
                      double move, double* xout, cudaStream_t st);
 

@@ -111,40 +111,210 @@ __device__ __forceinline__ double oc_new(double x, double dc, double dv, double 
   return fmax(0.0, fmax(x - move, fmin(1.0, fmin(x + move, be))));
 }
 
+// What the volume of the update needs per element.  The update of one element
+// is clamp(x sqrt(-dc / dv) / sqrt(lambda), lo, hi): t = x sqrt(-dc / dv) and
+// the limits do not depend on lambda, so the division and the square root
+// (about 12 FP64 instructions each on a part that issues 2 FP64 instructions
+// per clock and SM) are done once per element and not once per element and
+// multiplier.  lo = max(0, x - move), hi = min(1, x + move); a t that is NaN
+// (dc > 0) selects hi, as fmin / fmax do in oc_new.
+struct OcElem {
+  double t, lo, hi;
+};
+__device__ __forceinline__ OcElem oc_elem(double x, double dc, double dv, double move) {
+  OcElem e;
+  e.t = x * sqrt(-dc / dv);
+  e.t = e.t <= 0.0 ? 0.0 : e.t;  // -0 and negative products give lo, a NaN stays
+  e.lo = fmax(0.0, x - move);
+  e.hi = fmax(0.0, fmin(1.0, x + move));
+  return e;
+}
+// max(lo, min(hi, be)) on the bit patterns: every finite value here is >= 0,
+// where doubles order as their bits, and a NaN of either sign lies above hi.
+// Integer comparisons leave the FP64 pipe to the product and the sum.
+__device__ __forceinline__ double oc_clamp(double be, double lo, double hi, bool* inside) {
+  const unsigned long long b = __double_as_longlong(be), l = __double_as_longlong(lo), h = __double_as_longlong(hi);
+  *inside = b < h && b > l;
+  const double v = b < h ? be : hi;
+  return b < l || h < l ? lo : v;
+}
+
+// Block sums of NS values per thread in a fixed order: the block's totals go
+// to part[block * NS + q]; the last block (by ticket) returns true in all its
+// threads with the totals over the blocks, added in block order, in tot.
+template <int NS, typename A>
+__device__ __forceinline__ bool oc_block_totals(A (&acc)[NS], double* __restrict__ part, unsigned* ticket,
+                                                double* tot) {
+  __shared__ A sw[8][NS];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < NS; ++q) {
+    A v = acc[q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == (q & 31)) sw[wid][q] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < NS) {
+    double s = 0.0;
+    for (int w = 0; w < 8; ++w) s += (double)sw[w][threadIdx.x];
+    part[(long long)blockIdx.x * NS + threadIdx.x] = s;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  // the blocks in 256 / NS strided runs per value, then the runs in order
+  constexpr int RUNS = 256 / NS;
+  __shared__ double sr[NS][RUNS];
+  const int q = threadIdx.x % NS, run = threadIdx.x / NS;
+  if (run < RUNS) {
+    double s = 0.0;
+    for (unsigned b = run; b < gridDim.x; b += RUNS) s += ((volatile double*)part)[(long long)b * NS + q];
+    sr[q][run] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < NS) {
+    double s = 0.0;
+    for (int r = 0; r < RUNS; ++r) s += sr[threadIdx.x][r];
+    tot[threadIdx.x] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *ticket = 0u;
+  return true;
+}
+
+// Per-element arrays of the search (24 B written per element) and the bracket
+// of its root: the volume at kOcCand values of s = 1/sqrt(lambda), each twice
+// the one before from lambda = 1e9 down, in FP32 (the FP64 pipe is 64 times
+// narrower; the bracket is widened by a candidate on either side, so FP32's
+// 1e-6 does not decide anything).  With the Newton steps below the update of
+// 256x128x128 elements takes 0.69 ms; 16 passes that each evaluated 31
+// multipliers of the bisection in FP64 (5.8 ms a pass, two divisions and a
+// square root per multiplier) took 93.7 ms, with bitwise the same result.
+constexpr int kOcCand = 32;
+__global__ void __launch_bounds__(256) oc_prepare_kernel(const double* __restrict__ x, const double* __restrict__ dc,
+                                                         const double* __restrict__ dv, long long n, double move,
+                                                         double target, double* __restrict__ t,
+                                                         double* __restrict__ lo, double* __restrict__ hi,
+                                                         double* __restrict__ part, OcState* __restrict__ st) {
+  const float s0 = 3.1622776e-5f;  // 1 / sqrt(1e9)
+  float acc[kOcCand];
+#pragma unroll
+  for (int q = 0; q < kOcCand; ++q) acc[q] = 0.f;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+    const OcElem el = oc_elem(x[e], dc[e], dv[e], move);
+    t[e] = el.t;
+    lo[e] = el.lo;
+    hi[e] = el.hi;
+    const float l = (float)el.lo, h = (float)el.hi;
+    float be = (float)el.t * s0;
+#pragma unroll
+    for (int q = 0; q < kOcCand; ++q) {
+      acc[q] += fmaxf(l, fminf(h, be));  // NaN: h
+      be += be;
+    }
+  }
+  __shared__ double tot[kOcCand];
+  if (!oc_block_totals<kOcCand, float>(acc, part, &st->ticket, tot) || threadIdx.x != 0) return;
+  int k = 0;
+  while (k < kOcCand && !(tot[k] > target)) ++k;
+  const double s00 = 1.0 / sqrt(1e9);
+  auto at = [&](int q) { return q < 0 ? 0.0 : s00 * exp2((double)q); };
+  st->state = 0;
+  if (k == kOcCand) {  // no multiplier of the range reaches the target (or NaN)
+    st->state = 2;
+    return;
+  }
+  st->s_lo = at(k - 2);
+  st->s_hi = at(k + 1);
+  const double v0 = k > 0 ? tot[k - 1] : 0.0;
+  const double a = at(k - 1), b = at(k);
+  double s = a + (target - v0) / (tot[k] - v0) * (b - a);
+  if (!(s > st->s_lo && s < st->s_hi)) s = 0.5 * (st->s_lo + st->s_hi);
+  st->s = s;
+}
+
+// One step of the search for V(s) = target: V and its slope at s in FP64, then
+// a Newton step kept inside the bracket (V is piecewise linear and does not
+// fall with s).  Done when the step is below 1e-10 s: the root is then
+// s + step to the rounding of V itself, since between s and the root the
+// elements change their branch by less than 1e-10 of their value.
+__global__ void __launch_bounds__(256) oc_step_kernel(const double* __restrict__ t, const double* __restrict__ lo,
+                                                      const double* __restrict__ hi, long long n, double target,
+                                                      double* __restrict__ part, OcState* __restrict__ st) {
+  if (*((volatile int*)&st->state) != 0) return;
+  const double s = *((volatile double*)&st->s);
+  double acc[2] = {0.0, 0.0};
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+    const double te = t[e];
+    bool inside;
+    acc[0] += oc_clamp(te * s, lo[e], hi[e], &inside);
+    if (inside) acc[1] += te;
+  }
+  __shared__ double tot[2];
+  if (!oc_block_totals<2, double>(acc, part, &st->ticket, tot) || threadIdx.x != 0) return;
+  const double V = tot[0], slope = tot[1];
+  if (V > target) st->s_hi = s;
+  else st->s_lo = s;
+  const double sn = s + (target - V) / slope;
+  if (fabs(sn - s) <= 1e-10 * s) {
+    st->root = sn;
+    st->state = 1;
+  } else {
+    st->s = (sn > st->s_lo && sn < st->s_hi) ? sn : 0.5 * (st->s_lo + st->s_hi);
+  }
+}
+
+void launch_oc_prepare(const double* x, const double* dc, const double* dv, long long n, double move, double target,
+                       double* t, double* lo, double* hi, double* part, OcState* st, int nblocks, cudaStream_t s) {
+  oc_prepare_kernel<<<nblocks, 256, 0, s>>>(x, dc, dv, n, move, target, t, lo, hi, part, st);
+}
+void launch_oc_step(const double* t, const double* lo, const double* hi, long long n, double target, double* part,
+                    OcState* st, int nblocks, cudaStream_t s) {
+  oc_step_kernel<<<nblocks, 256, 0, s>>>(t, lo, hi, n, target, part, st);
+}
+
 // Sum over elements of x_new(lambda_q) for nlam candidate multipliers; block
-// partials [block][nlam] are summed in block order by the caller's finalize.
-__global__ void oc_volumes_kernel(const double* __restrict__ x, const double* __restrict__ dc,
-                                  const double* __restrict__ dv, long long n, const double* __restrict__ lam, int nlam,
-                                  double move, double* __restrict__ partials) {
+// partials [block][32] are summed in block order by the caller.  Only for
+// volumes without a root in the search's range (a target that no multiplier
+// reaches, NaN input).
+__global__ void oc_volumes_kernel(const double* __restrict__ t, const double* __restrict__ lo,
+                                  const double* __restrict__ hi, long long n, const double* __restrict__ lam, int nlam,
+                                  double* __restrict__ partials) {
   __shared__ double sl[32];
   __shared__ double sw[8][32];
-  if (threadIdx.x < nlam) sl[threadIdx.x] = lam[threadIdx.x];
+  if (threadIdx.x < nlam) sl[threadIdx.x] = 1.0 / sqrt(lam[threadIdx.x]);
   __syncthreads();
   double acc[32];
 #pragma unroll
   for (int q = 0; q < 32; ++q) acc[q] = 0.0;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const double xe = x[e], de = dc[e], ve = dv[e];
+    const double te = t[e], l = lo[e], h = hi[e];
+    bool inside;
 #pragma unroll
     for (int q = 0; q < 32; ++q)
-      if (q < nlam) acc[q] += oc_new(xe, de, ve, sl[q], move);
+      if (q < nlam) acc[q] += oc_clamp(te * sl[q], l, h, &inside);
   }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
   for (int q = 0; q < 32; ++q) {
-    double t = warp_sum(acc[q]);
-    if (lane == q) sw[wid][q] = t;
+    double v = warp_sum(acc[q]);
+    if (lane == q) sw[wid][q] = v;
   }
   __syncthreads();
   if (threadIdx.x < nlam) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sw[w][threadIdx.x];
-    partials[(long long)blockIdx.x * 32 + threadIdx.x] = t;
+    double v = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += sw[w][threadIdx.x];
+    partials[(long long)blockIdx.x * 32 + threadIdx.x] = v;
   }
 }
-void launch_oc_volumes(const double* x, const double* dc, const double* dv, long long n, const double* lam, int nlam,
-                       double move, double* partials, int nblocks, cudaStream_t st) {
-  oc_volumes_kernel<<<nblocks, 256, 0, st>>>(x, dc, dv, n, lam, nlam, move, partials);
+void launch_oc_volumes(const double* t, const double* lo, const double* hi, long long n, const double* lam, int nlam,
+                       double* partials, int nblocks, cudaStream_t st) {
+  oc_volumes_kernel<<<nblocks, 256, 0, st>>>(t, lo, hi, n, lam, nlam, partials);
 }
 
 __global__ void oc_apply_kernel(const double* __restrict__ x, const double* __restrict__ dc, const double* __restrict__ dv,
