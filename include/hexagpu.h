@@ -258,7 +258,7 @@ int hexa_filter(hexa_ctx* ctx, const hexa_grid* g, const double* rho_in, double 
  * device memory where they filter -- code running on its own stream while
  * another stream of its application is being captured into a CUDA graph, or
  * hosts whose own pool owns the device-memory budget.  All scratch lives in
- * one fixed device array inside the library (about 15 MB, held by every GPU
+ * one fixed device array inside the library (about 10.5 MB, held by every GPU
  * that loads the library until exit), so the grid may have at most
  * HEXA_NOALLOC_MAX_NODES nodes; larger grids return HEXA_ERR_TOO_LARGE.
  * rho_in and rho_out must be device pointers on the current device (host

@@ -794,7 +794,7 @@ int batch_filter_t(Ctx& c, int count, const hexa_grid* grids, const double* cons
       cudaMemcpyAsync(out64 + eoff[i], rho64 + eoff[i], sizeof(double) * g[i].nelem(), cudaMemcpyDeviceToDevice, c.st);
       continue;
     }
-    launch_helm_extract<T>(g[i], x + noff[i], outT + eoff[i], c.st);
+    launch_helm_mean<T, T>(g[i], x + noff[i], outT + eoff[i], c.st);
     c.launches++;
     if constexpr (sizeof(T) == 8) {
       cudaMemcpyAsync(out64 + eoff[i], outT + eoff[i], sizeof(double) * g[i].nelem(), cudaMemcpyDeviceToDevice, c.st);

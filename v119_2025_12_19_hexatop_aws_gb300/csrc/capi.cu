@@ -605,92 +605,75 @@ int hexa_solve_multi_rhs(hexa_ctx* h, const hexa_grid* g, const hexa_bc* bc, con
 
 }  // extern "C"
 
-// The filter's PCG on a device density of type T (GPUHelmholtz.jl:180-260):
-// writes the filtered element field into outT, or sets *zero and leaves outT
+// The filter's PCG in precision T on a device density (GPUHelmholtz.jl:180-260):
+// writes the filtered element field into out, or sets *zero and leaves out
 // alone when the right-hand side is zero (the reference returns its input
-// unchanged, GPUHelmholtz.jl:203-206).
-template <typename T>
-static int filter_run(hexa_ctx* h, const Grid& G, const T* rho, const HelmK& K, double tol, int max_iter, T* outT,
+// unchanged, GPUHelmholtz.jl:203-206).  The zero test rides on the scalars
+// that come back after the first ten iterations, whose launches then return
+// at once.
+template <typename T, typename TI, typename TO>
+static int filter_run(hexa_ctx* h, const Grid& G, const TI* rho, const HelmK& K, double tol, int max_iter, TO* out,
                       hexa_filter_stats* st, bool* zero) {
   Ctx& c = h->c;
   const long long nn = G.nnode();
   const char* tg = sizeof(T) == 8 ? "h64_" : "h32_";
   auto nm = [&](const char* s) { return std::string(tg) + s; };
-  T* b = c.vec<T>(nm("b"), nn);
   T* x = c.vec<T>(nm("x"), nn);
   T* r = c.vec<T>(nm("r"), nn);
-  T* z = c.vec<T>(nm("z"), nn);
-  T* p = c.vec<T>(nm("p"), nn);
+  T* pa = c.vec<T>(nm("p"), nn);
+  T* pb = c.vec<T>(nm("p2"), nn);
   T* q = c.vec<T>(nm("q"), nn);
-  T* dinv = c.vec<T>(nm("dinv"), nn);
-  if (!b || !x || !r || !z || !p || !q || !dinv) return HEXA_ERR_NOMEM;
+  if (!x || !r || !pa || !pb || !q || !c.ensure_partials(kHelmPartials)) return HEXA_ERR_NOMEM;
   *zero = false;
-  launch_helm_rhs<T>(G, rho, (T)K.rhs_scale, b, c.st);
-  launch_helm_dinv<T>(G, K, dinv, c.st);
-  c.launches += 2;
-  RedArgs rd;
-  rd.partials = c.partials;
-  rd.ticket = c.ticket;
-  rd.s = c.s;
-  rd.dst = c.dscal + 20;
-  rd.op = FIN_STORE;
-  rd.nsum = 1;
-  launch_dot<T>(b, b, (const T*)nullptr, (const T*)nullptr, nn, rd, kRed, nullptr, c.st);
-  c.launches++;
-  cudaMemcpyAsync(c.hscal + 20, c.dscal + 20, sizeof(double), cudaMemcpyDeviceToHost, c.st);
-  cudaStreamSynchronize(c.st);
-  const double bnorm = std::sqrt(c.hscal[20]);
-  if (bnorm == 0.0) {
-    *zero = true;
-    st->iterations = 0;
-    st->relres = 0.0;
-    st->solve_ms = 0.0;
-    return HEXA_OK;
-  }
+  const HelmPlan plan = helm_plan(G);
   PcgScalars hs;
   std::memset(&hs, 0, sizeof(hs));
   hs.tol = tol;
   hs.max_iter = max_iter;
   hs.cadence = -10;
   hs.no_div = 1;
-  hs.bnorm = bnorm;
   hs.best_rel = INFINITY;
   *c.hs = hs;
   cudaMemcpyAsync(c.s, c.hs, sizeof(PcgScalars), cudaMemcpyHostToDevice, c.st);
-  launch_fill<T>(x, T(0), nn, c.st);
-  launch_copy<T>(r, b, nn, c.st);
-  c.launches += 2;
+  RedArgs rd;
+  rd.partials = c.partials;
+  rd.ticket = c.ticket;
   rd.s = c.s;
-  rd.op = FIN_INIT_RZ;
-  launch_jacobi_precond<T>(z, r, dinv, nn, rd, kRed, nullptr, c.st);
-  launch_copy<T>(p, z, nn, c.st);
-  c.launches += 2;
+  rd.dst = nullptr;
+  rd.op = FIN_HELM_INIT;
+  rd.nsum = 2;
+  RedArgs ra = rd, rb = rd;
+  ra.op = FIN_PCG_ALPHA;
+  ra.nsum = 1;
+  rb.op = FIN_PCG_RES;
+  launch_helm_init<T, TI>(G, K, rho, r, rd, c.st);
+  c.launches++;
   cudaEventRecord(c.ev[0], c.st);
-  const int* halt = &c.s->halt;
-  const int hblocks = (int)std::min<long long>((nn + 255) / 256, 152 * 8);
   while (true) {
     for (int it = 0; it < 10; ++it) {
-      RedArgs ra = rd;
-      ra.op = FIN_PCG_ALPHA;
-      launch_helm_apply_dot<T>(G, K, p, q, ra, hblocks, halt, c.st);
-      RedArgs rb = rd;
-      rb.op = FIN_PCG_RES;
-      rb.nsum = 2;
-      launch_pcg_update<T>(x, r, z, p, q, dinv, nn, rb, kRed, c.s, c.st);
-      launch_p_update<T>(p, z, nn, c.s, c.st);
-      c.launches += 3;
+      launch_helm_dir<T>(G, plan, K, r, pa, pb, q, ra, c.s, c.st);
+      launch_helm_update<T>(G, x, r, pb, q, rb, c.s, c.st);
+      std::swap(pa, pb);
     }
+    c.launches += 20;
     cudaMemcpyAsync(c.hs, c.s, sizeof(PcgScalars), cudaMemcpyDeviceToHost, c.st);
     if (cudaStreamSynchronize(c.st) != cudaSuccess) return HEXA_ERR_CUDA;
     if (c.hs->halt) break;
+  }
+  if (c.hs->status == 5) {
+    *zero = true;
+    st->iterations = 0;
+    st->relres = 0.0;
+    st->solve_ms = 0.0;
+    return HEXA_OK;
   }
   if (c.hs->status == 2 || c.hs->status == 4) {
     // a NaN residual or a breakdown of p.Ap: the reference's loop goes on with
     // alpha = rho / p.Ap non-finite and returns a NaN field (its callers test
     // for that, TopOpt.jl:360-363), so the output is NaN here too
-    launch_fill<T>(outT, std::numeric_limits<T>::quiet_NaN(), G.nelem(), c.st);
+    launch_fill<TO>(out, std::numeric_limits<TO>::quiet_NaN(), G.nelem(), c.st);
   } else {
-    launch_helm_extract<T>(G, x, outT, c.st);
+    launch_helm_mean<T, TO>(G, x, out, c.st);
   }
   c.launches++;
   cudaEventRecord(c.ev[1], c.st);
@@ -706,29 +689,11 @@ static int filter_run(hexa_ctx* h, const Grid& G, const T* rho, const HelmK& K, 
 template <typename T>
 static int filter_t(hexa_ctx* h, const Grid& G, const double* rho_d, const HelmK& K, double tol, int max_iter,
                     double* out_d, hexa_filter_stats* st) {
-  Ctx& c = h->c;
-  const long long ne = G.nelem();
-  const char* tg = sizeof(T) == 8 ? "h64_" : "h32_";
-  T* rho = c.vec<T>(std::string(tg) + "rho", ne);
-  T* outT = c.vec<T>(std::string(tg) + "out", ne);
-  if (!rho || !outT) return HEXA_ERR_NOMEM;
-  if constexpr (sizeof(T) == 8) cudaMemcpyAsync(rho, rho_d, ne * sizeof(double), cudaMemcpyDeviceToDevice, c.st);
-  else {
-    launch_convert<float, double>(rho, rho_d, ne, c.st);
-    c.launches++;
-  }
   bool zero = false;
-  const int rc = filter_run<T>(h, G, rho, K, tol, max_iter, outT, st, &zero);
-  if (rc != HEXA_OK) return rc;
-  if (zero) {
-    cudaMemcpyAsync(out_d, rho_d, ne * sizeof(double), cudaMemcpyDeviceToDevice, c.st);
-  } else if constexpr (sizeof(T) == 8) {
-    cudaMemcpyAsync(out_d, outT, ne * sizeof(double), cudaMemcpyDeviceToDevice, c.st);
-  } else {
-    launch_convert<double, float>(out_d, outT, ne, c.st);
-    c.launches++;
-  }
-  return HEXA_OK;
+  const int rc = filter_run<T, double, double>(h, G, rho_d, K, tol, max_iter, out_d, st, &zero);
+  if (rc == HEXA_OK && zero && out_d != rho_d)
+    cudaMemcpyAsync(out_d, rho_d, G.nelem() * sizeof(double), cudaMemcpyDeviceToDevice, h->c.st);
+  return rc;
 }
 
 extern "C" {
@@ -875,25 +840,13 @@ int hexa_update_density(hexa_ctx* h, const hexa_grid* g, float* density, const f
     std::memset(&fs, 0, sizeof(fs));
     bool zero = false;
     int rc;
-    if (p->filter_precision == HEXA_PREC_FP64) {
-      double* p64 = c.vec<double>("h64_rho", ne);
-      double* o64 = c.vec<double>("h64_out", ne);
-      float* filt = c.vec<float>("ud_filt", ne);
-      if (!p64 || !o64 || !filt) return set_err(h, HEXA_ERR_NOMEM, "density update: out of device memory");
-      launch_convert<double, float>(p64, prop, ne, c.st);
-      c.launches++;
-      rc = filter_run<double>(h, G, p64, K, p->filter_tolerance, p->filter_max_iter, o64, &fs, &zero);
-      if (rc == HEXA_OK && !zero) {
-        launch_convert<float, double>(filt, o64, ne, c.st);
-        c.launches++;
-        src = filt;
-      }
-    } else {
-      float* filt = c.vec<float>("h32_out", ne);
-      if (!filt) return set_err(h, HEXA_ERR_NOMEM, "density update: out of device memory");
-      rc = filter_run<float>(h, G, prop, K, p->filter_tolerance, p->filter_max_iter, filt, &fs, &zero);
-      if (rc == HEXA_OK && !zero) src = filt;
-    }
+    float* filt = c.vec<float>("ud_filt", ne);
+    if (!filt) return set_err(h, HEXA_ERR_NOMEM, "density update: out of device memory");
+    if (p->filter_precision == HEXA_PREC_FP64)
+      rc = filter_run<double, float, float>(h, G, prop, K, p->filter_tolerance, p->filter_max_iter, filt, &fs, &zero);
+    else
+      rc = filter_run<float, float, float>(h, G, prop, K, p->filter_tolerance, p->filter_max_iter, filt, &fs, &zero);
+    if (rc == HEXA_OK && !zero) src = filt;
     if (rc != HEXA_OK) return set_err(h, rc, c.err.empty() ? "density update: filter failed" : c.err);
     st.filter_time = fs.solve_ms / 1e3;
     st.filter_iters = fs.iterations;

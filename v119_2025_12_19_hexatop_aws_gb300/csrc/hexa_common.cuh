@@ -73,7 +73,7 @@ struct PcgScalars {
   double tol;
   double dtmp[6];   // scratch reduction results
   int halt;         // nonzero: every kernel of the iteration returns at once
-  int status;       // 0 running, 1 converged, 2 nan/inf, 3 diverged, 4 breakdown (|pAp|<1e-20)
+  int status;       // 0 running, 1 converged, 2 nan/inf, 3 diverged, 4 breakdown (|pAp|<1e-20), 5 zero rhs (filter)
   int iter;         // completed iterations
   int max_iter;
   int cadence;      // test convergence when iter==1 or iter%cadence==0
@@ -92,6 +92,7 @@ enum FinalizeOp {
   FIN_INIT_RZ = 6,      // rz = sum0
   FIN_BLOCK_RES = 7,    // nsum column norms ||R_j||^2 (to dst when given); rr = max; test, iter++
   FIN_PCG_RES_MG = 8,   // FIN_PCG_RES with sum1 = r_new.z_old kept for FIN_PCG_BETA_RZ
+  FIN_HELM_INIT = 10,   // bnorm = sqrt(sum0), rz = sum1; a zero right-hand side halts (status 5)
   FIN_PCG_BETA_RZ = 9,  // rz_new = sum0; flexible beta = (rz_new - r_new.z_old) / rz
 };
 
@@ -134,7 +135,16 @@ __device__ __forceinline__ void finalize_scalars(const RedArgs& r, const double*
       // GPUSolver.jl:374 stops on the absolute test |p.Ap| < 1e-20, which ends
       // tight solves of unit-load problems early; for the SPD (K + sigma I)
       // only non-positive (or NaN) curvature is a breakdown here.
-      if (!(tot[0] > 0.0)) {
+      if (tot[0] == 0.0 && s->rz == 0.0 && s->cadence < 0) {
+        // the filter's residual became exactly zero (a constant density can do
+        // that in one iteration): converged, seen at the loop's next test
+        const int cad = -s->cadence;
+        s->iter = min((s->iter + cad - 1) / cad * cad, s->max_iter);
+        s->relres = 0.0;
+        s->status = 1;
+        s->halt = 1;
+        s->alpha = 0.0;
+      } else if (!(tot[0] > 0.0)) {
         s->status = 4;
         s->halt = 1;
         s->alpha = 0.0;
@@ -198,6 +208,11 @@ __device__ __forceinline__ void finalize_scalars(const RedArgs& r, const double*
     }
     case FIN_INIT_RZ:
       s->rz = tot[0];
+      break;
+    case FIN_HELM_INIT:
+      s->bnorm = sqrt(tot[0]);
+      s->rz = tot[1];
+      if (s->bnorm == 0.0) s->halt = 1, s->status = 5;
       break;
     case FIN_BLOCK_RES: {
       double mx = 0.0;

@@ -137,15 +137,37 @@ struct HelmK {
   double A[8][8];  // R^2 Ke + Me, corner order dx + 2dy + 4dz
   double rhs_scale; // vol/8
 };
+// One grid: the Jacobi-PCG of the filter in two launches per iteration; s->iter
+// == 0 marks the first (no previous direction, x not yet written).
+// The preconditioner is z = 2^faces r (D^-1 up to a constant factor).
+// r = b = rhs_scale * sum of the densities around a node; sums b.b, b.z
+template <typename T, typename TI>
+void launch_helm_init(const Grid& g, const HelmK& K, const TI* rho, T* r, const RedArgs& red, cudaStream_t st);
+// pn = z + beta po, q = A pn, sum pn.q (po and pn are different vectors)
+struct HelmPlan {
+  int tx, ty, threads;  // columns of a tile, threads of a CTA
+  int ntx, nty, kchunk; // tiles per axis, layers per item
+  long long items;
+  int blocks;
+};
+HelmPlan helm_plan(const Grid& g);
+template <typename T>
+void launch_helm_dir(const Grid& g, const HelmPlan& pl, const HelmK& K, const T* r, const T* po, T* pn, T* q, const RedArgs& red,
+                     const PcgScalars* s, cudaStream_t st);
+// x += alpha p, r -= alpha q; sums r.r, r.z
+template <typename T>
+void launch_helm_update(const Grid& g, T* x, T* r, const T* p, const T* q, const RedArgs& red, const PcgScalars* s,
+                        cudaStream_t st);
+// element mean of psi
+template <typename T, typename TO>
+void launch_helm_mean(const Grid& g, const T* psi, TO* out, cudaStream_t st);
+// doubles of reduction partials that the passes above need at most
+constexpr int kHelmPartials = 2432;
+// vectors of the batched form
 template <typename T>
 void launch_helm_rhs(const Grid& g, const T* rho, T scale, T* b, cudaStream_t st);
 template <typename T>
-void launch_helm_apply_dot(const Grid& g, const HelmK& K, const T* x, T* y, const RedArgs& red,
-                           int nblocks, const int* halt, cudaStream_t st);
-template <typename T>
 void launch_helm_dinv(const Grid& g, const HelmK& K, T* dinv, cudaStream_t st);
-template <typename T>
-void launch_helm_extract(const Grid& g, const T* psi, T* rho_out, cudaStream_t st);
 
 // ------------------------------------------------------------------ SIMP/OC
 void launch_simp_factors(const double* rho, double Emin, double E0, double penal, double* fac,

@@ -7,8 +7,8 @@
 // global-mode capture an allocation is a prohibited call on every thread), or
 // hosts that hand the whole device-memory budget to their own pool and forbid
 // other allocations mid-run.  This entry point takes device arrays for its
-// input and output and keeps all of its scratch -- the six work vectors and
-// the inverse diagonal of the Jacobi-PCG, the reduction partials, the ticket
+// input and output and keeps all of its scratch -- the five work vectors of
+// the Jacobi-PCG, the reduction partials, the ticket
 // counter and the iteration scalars -- in one file-scope device array of fixed
 // size, so it allocates nothing: no cudaMalloc, no cudaFree, no allocating
 // library call.
@@ -24,7 +24,7 @@
 // not refused because the application is capturing elsewhere, and restores the
 // thread's mode before it returns.
 //
-// The array holds HEXA_NOALLOC_MAX_NODES grid nodes (about 15 MB); every GPU
+// The array holds HEXA_NOALLOC_MAX_NODES grid nodes (about 10.5 MB); every GPU
 // that loads the library keeps it until the process exits.  Every call shares
 // it and it keeps the last call's contents, so each call clears what must
 // start at zero (the ticket counter) and rewrites everything else before use;
@@ -40,6 +40,7 @@
 #include <cstring>
 #include <limits>
 #include <mutex>
+#include <utility>
 
 #include "../../include/hexagpu.h"
 #include "element.h"
@@ -50,10 +51,9 @@ namespace {
 using namespace hexa;
 
 constexpr long long kMaxNodes = HEXA_NOALLOC_MAX_NODES;
-constexpr int kVecs = 7;                // b, x, r, z, p, q, dinv
+constexpr int kVecs = 5;                // x, r, p (two, alternating), q
 constexpr long long kHeader = 4224;      // doubles: scalars, ticket, results, partials
 constexpr long long kScratchDoubles = kHeader + kVecs * kMaxNodes;
-constexpr int kRedBlocksNA = 152 * 4;    // grid of the reducing vector passes
 constexpr int kMaxDevices = 64;
 
 // The scratch.  In host code this name is a host-side stand-in, never a device
@@ -155,72 +155,58 @@ extern "C" int hexa_filter_noalloc(const hexa_grid* g, const double* rho_in, dou
   double* partials = base + 128;
   const long long nn = G.nnode();
   double* vec = base + kHeader;
-  double *b = vec, *x = vec + kMaxNodes, *r = vec + 2 * kMaxNodes, *z = vec + 3 * kMaxNodes,
-         *p = vec + 4 * kMaxNodes, *q = vec + 5 * kMaxNodes, *dinv = vec + 6 * kMaxNodes;
+  double *x = vec, *r = vec + kMaxNodes, *pa = vec + 2 * kMaxNodes, *pb = vec + 3 * kMaxNodes,
+         *q = vec + 4 * kMaxNodes;
+  static_assert(kHelmPartials <= kHeader - 128, "reduction partials exceed their place in the scratch");
+  const HelmPlan plan = helm_plan(G);
 
   // the previous call's contents stay behind: the ticket must start at zero
   cudaMemsetAsync(ticket, 0, sizeof(unsigned), st);
-  launch_helm_rhs<double>(G, rho_in, K.rhs_scale, b, st);
-  launch_helm_dinv<double>(G, K, dinv, st);
+  PcgScalars hs;
+  std::memset(&hs, 0, sizeof(hs));
+  hs.tol = tol;
+  hs.max_iter = max_iter;
+  hs.cadence = -10;
+  hs.no_div = 1;
+  hs.best_rel = INFINITY;
+  cudaMemcpyAsync(s, &hs, sizeof(PcgScalars), cudaMemcpyHostToDevice, st);
   RedArgs rd;
   rd.partials = partials;
   rd.ticket = ticket;
   rd.s = s;
-  rd.dst = result;
-  rd.op = FIN_STORE;
-  rd.nsum = 1;
-  launch_dot<double>(b, b, (const double*)nullptr, (const double*)nullptr, nn, rd, kRedBlocksNA, nullptr, st);
-  double bb = 0.0;
-  cudaMemcpyAsync(&bb, result, sizeof(double), cudaMemcpyDeviceToHost, st);
-  if (cudaStreamSynchronize(st) != cudaSuccess) {
-    cudaGetLastError();
-    return HEXA_ERR_CUDA;
-  }
+  rd.dst = nullptr;
+  rd.op = FIN_HELM_INIT;
+  rd.nsum = 2;
+  launch_helm_init<double, double>(G, K, rho_in, r, rd, st);
   hexa_filter_stats out;
   std::memset(&out, 0, sizeof(out));
-  const double bnorm = std::sqrt(bb);
-  if (bnorm == 0.0) {  // GPUHelmholtz.jl:203-206: the input comes back unchanged
-    cudaMemcpyAsync(rho_out, rho_in, sizeof(double) * G.nelem(), cudaMemcpyDeviceToDevice, st);
-  } else {
-    PcgScalars hs;
-    std::memset(&hs, 0, sizeof(hs));
-    hs.tol = tol;
-    hs.max_iter = max_iter;
-    hs.cadence = -10;
-    hs.no_div = 1;
-    hs.bnorm = bnorm;
-    hs.best_rel = INFINITY;
-    cudaMemcpyAsync(s, &hs, sizeof(PcgScalars), cudaMemcpyHostToDevice, st);
-    launch_fill<double>(x, 0.0, nn, st);
-    launch_copy<double>(r, b, nn, st);
-    rd.op = FIN_INIT_RZ;
-    launch_jacobi_precond<double>(z, r, dinv, nn, rd, kRedBlocksNA, nullptr, st);
-    launch_copy<double>(p, z, nn, st);
-    const int hblocks = (int)std::min<long long>((nn + 255) / 256, 152 * 8);
-    for (int guard = 0; guard <= max_iter / 10 + 1; ++guard) {
-      for (int it = 0; it < 10; ++it) {
-        RedArgs ra = rd;
-        ra.op = FIN_PCG_ALPHA;
-        launch_helm_apply_dot<double>(G, K, p, q, ra, hblocks, &s->halt, st);
-        RedArgs rb = rd;
-        rb.op = FIN_PCG_RES;
-        rb.nsum = 2;
-        launch_pcg_update<double>(x, r, z, p, q, dinv, nn, rb, kRedBlocksNA, s, st);
-        launch_p_update<double>(p, z, nn, s, st);
-      }
-      cudaMemcpyAsync(&hs, s, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st);
-      if (cudaStreamSynchronize(st) != cudaSuccess) {
-        cudaGetLastError();
-        return HEXA_ERR_CUDA;
-      }
-      if (hs.halt) break;
+  for (int guard = 0; guard <= max_iter / 10 + 1; ++guard) {
+    for (int it = 0; it < 10; ++it) {
+      RedArgs ra = rd, rb = rd;
+      ra.op = FIN_PCG_ALPHA;
+      ra.nsum = 1;
+      rb.op = FIN_PCG_RES;
+      launch_helm_dir<double>(G, plan, K, r, pa, pb, q, ra, s, st);
+      launch_helm_update<double>(G, x, r, pb, q, rb, s, st);
+      std::swap(pa, pb);
     }
+    cudaMemcpyAsync(&hs, s, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) {
+      cudaGetLastError();
+      return HEXA_ERR_CUDA;
+    }
+    if (hs.halt) break;
+  }
+  if (hs.status == 5) {  // zero right-hand side (GPUHelmholtz.jl:203-206): the input comes back unchanged
+    if (rho_out != rho_in)
+      cudaMemcpyAsync(rho_out, rho_in, sizeof(double) * G.nelem(), cudaMemcpyDeviceToDevice, st);
+  } else {
     if (hs.status == 2 || hs.status == 4) {
       // a NaN residual or a breakdown of p.Ap gives a NaN field, as hexa_filter
       // and the reference's loop do (its callers test for it, TopOpt.jl:360-363)
       launch_fill<double>(rho_out, std::numeric_limits<double>::quiet_NaN(), G.nelem(), st);
     } else {
-      launch_helm_extract<double>(G, x, rho_out, st);
+      launch_helm_mean<double, double>(G, x, rho_out, st);
     }
     out.iterations = hs.iter;
     out.relres = hs.relres;
