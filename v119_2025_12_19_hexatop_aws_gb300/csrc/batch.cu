@@ -205,7 +205,8 @@ int batch_levels(const Grid& g, uint32_t faces, int requested) {
 }
 
 // Buffers, coarse factors, coarse diagonals and device tables of the batch
-// hierarchy; the operator tables use z-bricks of kchunk layers.
+// hierarchy; the finest level's operator tables use z-bricks of kchunk layers
+// (0: picked), the others what op_batch_plan picks.
 template <typename T>
 bool build_batch_mg(Ctx& c, BatchMG<T>& mg, const std::vector<Grid>& g0, const std::vector<uint32_t>& faces,
                     const std::vector<double>& sigma, const std::vector<int>& nlev, const T* fac0, int kchunk) {
@@ -294,7 +295,7 @@ bool build_batch_mg(Ctx& c, BatchMG<T>& mg, const std::vector<Grid>& g0, const s
   for (int l = 0; l < maxlev; ++l) {
     BLevel<T>& V = mg.L[l];
     if (V.smooth.n()) {
-      V.smooth.oblocks = op_batch_plan<T>(V.smooth.h.data(), V.smooth.n(), kchunk);
+      V.smooth.oblocks = op_batch_plan<T>(V.smooth.h.data(), V.smooth.n(), l == 0 ? kchunk : 0);
       V.smooth.vblocks = vec_batch_plan(V.smooth.h.data(), V.smooth.n(), 1, kBatchVecBlocks);
       V.prolong.vblocks = vec_batch_plan(V.prolong.h.data(), V.prolong.n(), 1, kBatchVecBlocks);
     }
@@ -478,7 +479,7 @@ int batch_problem(Ctx& c, int count, const hexa_grid* grids, const hexa_bc* bcs,
   }
   std::vector<int> nlev(count);
   for (int i = 0; i < count; ++i) nlev[i] = batch_levels(g0[i], faces[i], prm.mg_levels);
-  int kchunk = 16;
+  int kchunk = 0;  // picked by op_batch_plan unless tuned
   const std::string tkey = "batch/" + std::to_string(count) + "/" + std::to_string(nelem) + "/" + std::to_string(ndof);
   bool tuned = false;
   if (prm.autotune) {
@@ -487,13 +488,13 @@ int batch_problem(Ctx& c, int count, const hexa_grid* grids, const hexa_bc* bcs,
   }
   if (!build_batch_mg<T>(c, mg, g0, faces, sigma, nlev, fac32, kchunk)) return HEXA_ERR_NOMEM;
   if (prm.autotune && !tuned && mg.L[0].smooth.n()) {
-    // z-brick depth: time the fine-level batched Chebyshev sweep for 8, 16 and 32 layers
+    // z-brick depth: time the fine-level batched Chebyshev sweep for the picked depth and 8, 16 and 32 layers
     launch_fill<T>(zA, T(0), ndof, c.st);
     launch_fill<T>(r, T(0), ndof, c.st);
     c.launches += 2;
     double best = INFINITY;
-    int bestk = 16;
-    for (int kc : {8, 16, 32}) {
+    int bestk = 0;
+    for (int kc : {0, 8, 16, 32}) {
       DevTable t;
       t.h = mg.L[0].smooth.h;
       t.oblocks = op_batch_plan<T>(t.h.data(), t.n(), kc);

@@ -49,7 +49,7 @@ void launch_op(int mode, const OpArgs<T>& a, cudaStream_t st);
 bool op_take_wait_error(cudaStream_t st);
 template <typename T>
 long long op_num_blocks(const Grid& g, int kchunk);
-// node layers per work item so that every resident CTA gets ~8 items
+// node layers per work item (see op.cu)
 template <typename T>
 int op_pick_kchunk(const Grid& g);
 ModalK<float> modal_to_f32(const ModalK<double>& K);
@@ -274,7 +274,7 @@ struct BatchInst {
   int pad;
 };
 
-// Fills the operator tiling (z-bricks of kchunk node layers, 0 = 16) and the
+// Fills the operator tiling (z-bricks of kchunk node layers, 0 = picked) and the
 // block ranges of n instances (targeting the resident CTAs of the operator in
 // precision T); returns the grid size.
 template <typename T>

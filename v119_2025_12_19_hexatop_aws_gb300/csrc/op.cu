@@ -985,17 +985,6 @@ long long op_num_blocks(const Grid& g, int kchunk) {
   return (long long)tx * ty * nch;
 }
 
-template <typename T>
-int op_pick_kchunk(const Grid& g) {
-  int tx, ty, nch;
-  op_tiles<T>(g, 1, &tx, &ty, &nch);
-  const long long tiles = (long long)tx * ty;
-  const long long want = 8LL * resident_ctas<T>(OP_CHEB2);  // ~8 items per CTA
-  long long chunks = (want + tiles - 1) / tiles;
-  chunks = std::max<long long>(1, std::min<long long>(chunks, (g.NZ + 15) / 16));  // chunks of >= 16 layers
-  return (int)((g.NZ + chunks - 1) / chunks);
-}
-
 static int env_int(const char* name, int dflt) {
   const char* v = std::getenv(name);
   return (v && *v) ? std::atoi(v) : dflt;
@@ -1009,6 +998,39 @@ static int env_int(const char* name, int dflt) {
 static int op_form() {
   static const int form = env_int("HEXA_OP_FORM", 0);
   return form;
+}
+
+// Node layers that starting an item costs: two more layers are loaded and one
+// more element layer is multiplied.  FP32 items are bound by each layer's chain
+// of loads, exchange and barriers, FP64 items by FP64 issue (the start has no
+// transform back and no epilogue).
+template <typename T>
+constexpr double op_item_start() { return sizeof(T) == 8 ? 0.6 : 2.0; }
+
+// Layers per item: the chunking for which the CTA with the most items has the
+// fewest layers to run, starts included.  Small grids get chunks of one or two
+// layers and fill the SMs (a 24x12x12 grid is one tile: one CTA marching its 13
+// layers took 13.6 us, 13 CTAs of one layer 5 us); large ones keep long
+// chunks that divide evenly over the CTAs.
+template <typename T>
+int op_pick_kchunk(const Grid& g) {
+  int tx, ty, nch;
+  op_tiles<T>(g, 1, &tx, &ty, &nch);
+  const long long tiles = (long long)tx * ty, ctas = resident_ctas<T>(OP_CHEB2);
+  if (sizeof(T) == 4 && op_form() == 1) {  // the staged form fills its ring over an item's layers: at least 16
+    long long chunks = (8 * ctas + tiles - 1) / tiles;
+    chunks = std::max<long long>(1, std::min<long long>(chunks, (g.NZ + 15) / 16));
+    return (int)((g.NZ + chunks - 1) / chunks);
+  }
+  double best = 1e300;
+  int kbest = g.NZ;
+  for (int n = 1; n <= std::min(g.NZ, 64); ++n) {
+    const int kc = (g.NZ + n - 1) / n;
+    const long long items = tiles * ((g.NZ + kc - 1) / kc);
+    const double t = (double)((items + ctas - 1) / ctas) * (kc + op_item_start<T>());
+    if (t < best) best = t, kbest = kc;
+  }
+  return kbest;
 }
 
 static int tma_resident_ctas() {
@@ -1170,24 +1192,53 @@ __global__ void __launch_bounds__(32 * TYW, op_min_ctas<T>()) op_batch_kernel(co
   }
 }
 
+// Blocks of a batch: every instance gets one, the rest of the resident CTAs go
+// one by one to the instance whose blocks have the most items each (more
+// blocks than resident CTAs would run a second, nearly empty wave).  Returns
+// the most items of any block.
+static long long batch_blocks(const std::vector<long long>& items, long long ctas, std::vector<int>* blocks) {
+  const int n = (int)items.size();
+  blocks->assign(n, 1);
+  auto per = [&](int i) { return (items[i] + (*blocks)[i] - 1) / (*blocks)[i]; };
+  for (long long left = ctas - n; left > 0; --left) {
+    int w = 0;
+    for (int i = 1; i < n; ++i)
+      if (per(i) > per(w)) w = i;
+    if (per(w) <= 1) break;
+    ++(*blocks)[w];
+  }
+  long long most = 0;
+  for (int i = 0; i < n; ++i) most = std::max(most, per(i));
+  return most;
+}
+
 template <typename T>
 int op_batch_plan(BatchInst* in, int n, int kchunk) {
-  long long total = 0;
+  const long long ctas = resident_ctas<T>(OP_CHEB2);
   std::vector<long long> items(n);
-  const int kc = kchunk > 0 ? kchunk : 16;
-  for (int i = 0; i < n; ++i) {
-    BatchInst& b = in[i];
-    b.kchunk = std::max(1, std::min(kc, b.g.NZ));
-    op_tiles<T>(b.g, b.kchunk, &b.tiles_x, &b.tiles_y, &b.nchunks);
-    items[i] = (long long)b.tiles_x * b.tiles_y * b.nchunks;
-    total += items[i];
+  std::vector<int> blocks;
+  auto tile = [&](int kc) {
+    for (int i = 0; i < n; ++i) {
+      BatchInst& b = in[i];
+      b.kchunk = std::max(1, std::min(kc, b.g.NZ));
+      op_tiles<T>(b.g, b.kchunk, &b.tiles_x, &b.tiles_y, &b.nchunks);
+      items[i] = (long long)b.tiles_x * b.tiles_y * b.nchunks;
+    }
+  };
+  if (kchunk <= 0) {  // as op_pick_kchunk: the chunking whose fullest block has the fewest layers to run
+    double best = 1e300;
+    for (int kc : {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32}) {
+      tile(kc);
+      const double t = (double)batch_blocks(items, ctas, &blocks) * (kc + op_item_start<T>());
+      if (t < best) best = t, kchunk = kc;
+    }
   }
-  const double per = std::max(1.0, (double)total / std::max(1, resident_ctas<T>(OP_CHEB2)));
+  tile(kchunk);
+  batch_blocks(items, ctas, &blocks);
   int blk = 0;
   for (int i = 0; i < n; ++i) {
-    const long long want = (long long)std::ceil((double)items[i] / per);
     in[i].oblk0 = blk;
-    in[i].onblk = (int)std::max<long long>(1, std::min<long long>(items[i], want));
+    in[i].onblk = (int)std::min<long long>(items[i], blocks[i]);
     blk += in[i].onblk;
   }
   return blk;
