@@ -84,7 +84,7 @@ typedef struct hexa_solve_params {
   double jacobi_omega;
   int32_t cheb_ratio;         /* Chebyshev smoothing interval [lmax/cheb_ratio, lmax] of D^-1 A (10) */
   int32_t coarse_iters;       /* Jacobi-PCG iterations of the coarsest-level solve when that grid
-                                 has more than 640 DOFs (smaller ones are solved exactly, by the
+                                 has more than 2304 DOFs (smaller ones are solved exactly, by the
                                  dense inverse of their operator) */
   double inner_tol;           /* mixed: relative tolerance of each FP32 correction solve */
   int32_t max_outer;          /* mixed: maximum refinement steps */

@@ -332,8 +332,18 @@ void launch_batch_prolong_add(const BatchInst* in, int ninst, int nblocks, const
 template <typename T>
 void launch_batch_jacobi0(const BatchInst* in, int ninst, int nblocks, const T* fac, const ModalK<T>& K, int quirk,
                           T omega, const T* b, T* x, const PcgScalars* s, cudaStream_t st);
-// x = A^-1 b with a dense symmetric n x n inverse (exact coarsest-level solve),
-// for ncol right-hand sides n apart
+// Inverse of (K + sigma I) on a small grid's free DOFs (FP64 sweep on the
+// device): A np x np and panels 2 np x 32 + 1024 doubles of workspace
+// (np = dense_padded(n)), ke the FP64 24x24 element matrix on the device; out
+// gets n rows of dense_ld(n) values, zero at fixed DOFs; *flag != 0 when a
+// pivot was not positive.  Returns the number of launches.
+int dense_padded(long long n);
+int dense_ld(long long n);
+template <typename T>
+int launch_dense_inverse(const Grid& g, const Mask& m, const T* fac, const double* ke, double sigma, double* A,
+                         double* panels, int* flag, T* out, cudaStream_t st);
+// x = A^-1 b with the rows that launch_dense_inverse leaves (exact
+// coarsest-level solve), for ncol right-hand sides n apart
 template <typename T>
 void launch_dense_coarse(long long n, const T* A, const T* b, T* x, const int* halt, cudaStream_t st,
                          int ncol = 1);

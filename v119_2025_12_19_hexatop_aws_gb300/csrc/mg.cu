@@ -786,34 +786,222 @@ void launch_batch_coarse_pcg(const BatchInst* in, int ninst, const T* fac, const
   batch_coarse_pcg_kernel<T><<<ninst, 1024, 0, st>>>(in, fac, K, dinv, b, x, r, z, p, q, w, iters, s);
 }
 
-// Exact coarsest-level solve: x = A^-1 b with the dense symmetric inverse
-// (n x n, zero rows/columns at fixed DOFs).  CTA = 32 rows, 8 warps split the
-// columns; lane = row, so each column read is one coalesced 128-byte access.
-// blockIdx.y picks one of ncol right-hand sides (vectors n apart).
+// ------------------------------------------------ exact coarsest-level solve
+// The inverse of the coarsest operator, built in FP64 on the device once per
+// shift and applied as one dense matvec per V-cycle.  Building it costs n^3/2
+// FP64 multiply-adds (1911 DOFs: about 9 ms); the 30 Jacobi-PCG iterations that
+// it replaces took 0.99 ms a visit on one CTA (12x6x6 grid), the matvec takes
+// about 4 us.
+//
+// Storage: an np x np matrix (np = n rounded up to whole 32-blocks, the padding
+// an identity), lower triangle of 32x32 blocks.  Fixed DOFs are rows of the
+// identity.  Block by block the symmetric sweep
+//   A_kk <- -D, A_ik <- A_ik D, A_ij <- A_ij - A_ik D A_kj,  D = A_kk^-1
+// leaves -A^-1 after the last block; the pivot blocks of a positive definite
+// matrix are positive definite, so there is no pivoting, and a pivot that is
+// not positive raises the flag.
+constexpr int kSweep = 32;
+
 template <typename T>
-__global__ void __launch_bounds__(256) dense_coarse_kernel(int n, const T* __restrict__ A, const T* __restrict__ b,
-                                                           T* __restrict__ x, const int* halt) {
+__global__ void __launch_bounds__(128) dense_assemble_kernel(Grid g, Mask m, const T* __restrict__ fac,
+                                                             const double* __restrict__ ke, double sigma, int np,
+                                                             double* __restrict__ A) {
+  const int n = (int)g.ndof(), nn = n / 3;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < np - n) A[(long long)(n + t) * np + n + t] = 1.0;
+  if (t >= 27 * nn) return;
+  const int a = t / 27, d = t - 27 * a;  // node and neighbour
+  const int i = a % g.NX, j = (a / g.NX) % g.NY, k = a / (g.NX * g.NY);
+  const int di = d % 3 - 1, dj = (d / 3) % 3 - 1, dk = d / 9 - 1;
+  const int i2 = i + di, j2 = j + dj, k2 = k + dk;
+  if (i2 < 0 || i2 >= g.NX || j2 < 0 || j2 >= g.NY || k2 < 0 || k2 >= g.NZ) return;
+  const int b = i2 + g.NX * (j2 + g.NY * k2);
+  // corner dx + 2dy + 4dz -> the reference's local node (Mesh.jl:45-53)
+  const int ref[8] = {0, 1, 3, 2, 4, 5, 7, 6};
+  double v[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+  for (int o = 0; o < 8; ++o) {  // element whose corner o is node a
+    const int ox = o & 1, oy = (o >> 1) & 1, oz = o >> 2;
+    const int ei = i - ox, ej = j - oy, ek = k - oz;
+    const int bx = ox + di, by = oy + dj, bz = oz + dk;  // node b's corner in it
+    if (ei < 0 || ei >= g.nx || ej < 0 || ej >= g.ny || ek < 0 || ek >= g.nz) continue;
+    if (bx < 0 || bx > 1 || by < 0 || by > 1 || bz < 0 || bz > 1) continue;
+    const double f = (double)fac[ei + (long long)g.nx * (ej + (long long)g.ny * ek)];
+    const int ra = 3 * ref[o], rb = 3 * ref[bx + 2 * by + 4 * bz];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int e = 0; e < 3; ++e) v[c][e] = fma(f, ke[ra + c + 24 * (rb + e)], v[c][e]);
+  }
+  const unsigned fa = fixed_bits(g, m, i, j, k, a), fb = fixed_bits(g, m, i2, j2, k2, b);
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      const bool fixd = ((fa >> c) & 1u) || ((fb >> e) & 1u), diag = a == b && c == e;
+      A[(long long)(3 * a + c) * np + 3 * b + e] = fixd ? (diag ? 1.0 : 0.0) : v[c][e] + (diag ? sigma : 0.0);
+    }
+}
+
+// Block row I of the panel of pivot block K: P_I = A_IK (from the lower
+// triangle) and W_I = P_I D.  Every CTA inverts the pivot block itself (in
+// shared memory, by the scalar sweep; one launch instead of two).
+__global__ void __launch_bounds__(256) dense_panel_kernel(const double* __restrict__ A, int np, int K,
+                                                          double* __restrict__ P, double* __restrict__ W,
+                                                          double* __restrict__ Dout, int* __restrict__ flag) {
+  __shared__ double D[kSweep][kSweep + 1], S[kSweep][kSweep + 1];
+  const int tid = threadIdx.x, r = tid >> 3, c0 = (tid & 7) * 4, I = blockIdx.x;
+  const long long k0 = (long long)K * kSweep;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int c = c0 + q;
+    D[r][c] = r >= c ? A[(k0 + r) * np + k0 + c] : A[(k0 + c) * np + k0 + r];
+    if (I >= K) S[r][c] = A[((long long)I * kSweep + r) * np + k0 + c];
+    else S[c][r] = A[(k0 + r) * np + (long long)I * kSweep + c];  // above the diagonal: from its transpose
+  }
+  __syncthreads();
+  for (int p = 0; p < kSweep; ++p) {
+    const double piv = D[p][p];
+    if (tid == 0 && I == 0 && !(piv > 0.0)) *flag = 1;
+    const double inv = 1.0 / piv, t = D[r][p];
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = c0 + q;
+      const double s = D[p][c] * inv;
+      v[q] = r == p ? (c == p ? inv : s) : (c == p ? -t * inv : fma(-t, s, D[r][c]));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) D[r][c0 + q] = v[q];
+    __syncthreads();
+  }
+  double w[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int k = 0; k < kSweep; ++k) {
+    const double s = S[r][k];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) w[q] = fma(s, D[k][c0 + q], w[q]);
+  }
+  const long long o = ((long long)I * kSweep + r) * kSweep + c0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    P[o + q] = S[r][c0 + q];
+    W[o + q] = w[q];
+    if (I == K) Dout[r * kSweep + c0 + q] = D[r][c0 + q];
+  }
+}
+
+// Block (I, J), I >= J, of the sweep of pivot block K.
+__global__ void __launch_bounds__(256) dense_update_kernel(double* __restrict__ A, int np, int K,
+                                                           const double* __restrict__ P, const double* __restrict__ W,
+                                                           const double* __restrict__ D) {
+  const int I = blockIdx.y, J = blockIdx.x;
+  if (J > I) return;
+  __shared__ double Wi[kSweep][kSweep + 1], Pj[kSweep][kSweep + 1];
+  const int tid = threadIdx.x, r = tid >> 3, c0 = (tid & 7) * 4;
+  double* a = A + ((long long)I * kSweep + r) * np + (long long)J * kSweep + c0;
+  const long long oi = ((long long)I * kSweep + r) * kSweep + c0, oj = ((long long)J * kSweep + r) * kSweep + c0;
+  if (I == K || J == K) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      a[q] = I == J ? -D[r * kSweep + c0 + q]
+                    : (J == K ? W[oi + q] : W[((long long)J * kSweep + c0 + q) * kSweep + r]);
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) Wi[r][c0 + q] = W[oi + q], Pj[r][c0 + q] = P[oj + q];
+  __syncthreads();
+  double v[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = a[q];
+#pragma unroll 8
+  for (int k = 0; k < kSweep; ++k) {
+    const double w = Wi[r][k];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = fma(-w, Pj[c0 + q][k], v[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) a[q] = v[q];
+}
+
+// A^-1 in the solver's precision, rows of ld values, zero at fixed DOFs.
+template <typename T>
+__global__ void dense_store_kernel(Grid g, Mask m, const double* __restrict__ A, int np, int ld, T* __restrict__ out) {
+  const int n = (int)g.ndof();
+  const int r = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ld) return;
+  T v = T(0);
+  if (c < n) {
+    auto fixd = [&](int dof) {
+      const int nd = dof / 3;
+      return (fixed_bits(g, m, nd % g.NX, (nd / g.NX) % g.NY, nd / (g.NX * g.NY), nd) >> (dof % 3)) & 1u;
+    };
+    if (!fixd(r) && !fixd(c)) v = (T)(r >= c ? -A[(long long)r * np + c] : -A[(long long)c * np + r]);
+  }
+  out[(long long)r * ld + c] = v;
+}
+
+int dense_padded(long long n) { return (int)((n + kSweep - 1) / kSweep) * kSweep; }
+int dense_ld(long long n) { return (int)((n + 3) / 4) * 4; }
+
+template <typename T>
+int launch_dense_inverse(const Grid& g, const Mask& m, const T* fac, const double* ke, double sigma, double* A,
+                         double* panels, int* flag, T* out, cudaStream_t st) {
+  const int n = (int)g.ndof(), np = dense_padded(n), nb = np / kSweep, ld = dense_ld(n);
+  double *P = panels, *W = panels + (size_t)np * kSweep, *D = W + (size_t)np * kSweep;
+  cudaMemsetAsync(A, 0, sizeof(double) * (size_t)np * np, st);
+  cudaMemsetAsync(flag, 0, sizeof(int), st);
+  dense_assemble_kernel<T><<<(27 * (n / 3) + 127) / 128, 128, 0, st>>>(g, m, fac, ke, sigma, np, A);
+  for (int k = 0; k < nb; ++k) {
+    dense_panel_kernel<<<nb, 256, 0, st>>>(A, np, k, P, W, D, flag);
+    dense_update_kernel<<<dim3(nb, nb), 256, 0, st>>>(A, np, k, P, W, D);
+  }
+  dense_store_kernel<T><<<dim3((ld + 127) / 128, n), 128, 0, st>>>(g, m, A, np, ld, out);
+  return 2 * nb + 2;
+}
+
+// x = A^-1 b.  A warp takes a row: 16-byte loads along it, all independent, b
+// from shared memory (1911 DOFs in FP32: 14.6 MB out of L2).  blockIdx.y picks
+// one of ncol right-hand sides (vectors n apart).
+template <typename T>
+__global__ void __launch_bounds__(256) dense_coarse_kernel(int n, int ld, const T* __restrict__ A,
+                                                           const T* __restrict__ b, T* __restrict__ x,
+                                                           const int* halt) {
   if (halt && *((volatile const int*)halt)) return;
+  extern __shared__ __align__(16) unsigned char dense_smem[];
+  T* sb = reinterpret_cast<T*>(dense_smem);
   b += (long long)blockIdx.y * n;
   x += (long long)blockIdx.y * n;
-  __shared__ T part[8][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int row = blockIdx.x * 32 + lane;
-  T s = T(0);
-  if (row < n)
-    for (int j = w; j < n; j += 8) s = fma(A[(long long)j * n + row], b[j], s);
-  part[w][lane] = s;
+  for (int i = threadIdx.x; i < ld; i += 256) sb[i] = i < n ? b[i] : T(0);
   __syncthreads();
-  if (w == 0 && row < n) {
-    T t = T(0);
+  const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= n) return;
+  const T* a = A + (long long)row * ld;
+  T s[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll 8
+  for (int c = 4 * lane; c < ld; c += 128) {
+    T v[4], w[4];
+    if constexpr (sizeof(T) == 4) {
+      *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(a + c);
+      *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(sb + c);
+    } else {
+      reinterpret_cast<double2*>(v)[0] = reinterpret_cast<const double2*>(a + c)[0];
+      reinterpret_cast<double2*>(v)[1] = reinterpret_cast<const double2*>(a + c)[1];
+      reinterpret_cast<double2*>(w)[0] = reinterpret_cast<const double2*>(sb + c)[0];
+      reinterpret_cast<double2*>(w)[1] = reinterpret_cast<const double2*>(sb + c)[1];
+    }
 #pragma unroll
-    for (int q = 0; q < 8; ++q) t += part[q][lane];
-    x[row] = t;
+    for (int q = 0; q < 4; ++q) s[q] = fma(v[q], w[q], s[q]);
   }
+  T t = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) x[row] = t;
 }
 template <typename T>
 void launch_dense_coarse(long long n, const T* A, const T* b, T* x, const int* halt, cudaStream_t st, int ncol) {
-  dense_coarse_kernel<T><<<dim3((unsigned)((n + 31) / 32), (unsigned)ncol), 256, 0, st>>>((int)n, A, b, x, halt);
+  const int ld = dense_ld(n);
+  dense_coarse_kernel<T><<<dim3((unsigned)((n + 7) / 8), (unsigned)ncol), 256, sizeof(T) * ld, st>>>((int)n, ld, A, b, x,
+                                                                                                    halt);
 }
 
 #define INST(T)                                                                                     \
@@ -827,6 +1015,8 @@ void launch_dense_coarse(long long n, const T* A, const T* b, T* x, const int* h
   template void launch_coarse_pcg<T>(const Grid&, const Mask&, const T*, const ModalK<T>&, T, const T*, \
                                      const T*, T*, T*, T*, T*, T*, T*, int, const int*, cudaStream_t);     \
   template void launch_dense_coarse<T>(long long, const T*, const T*, T*, const int*, cudaStream_t, int); \
+  template int launch_dense_inverse<T>(const Grid&, const Mask&, const T*, const double*, double, double*, \
+                                       double*, int*, T*, cudaStream_t);                                   \
   template void launch_batch_restrict<T>(const BatchInst*, int, int, const T*, T*, const PcgScalars*,     \
                                          cudaStream_t);                                                   \
   template void launch_batch_prolong_add<T>(const BatchInst*, int, int, const T*, T*, const PcgScalars*,  \

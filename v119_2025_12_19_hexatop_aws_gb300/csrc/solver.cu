@@ -193,13 +193,15 @@ void op(Ctx& c, int mode, const OpArgs<T>& a) {
 }
 
 // Number of levels: requested, or automatic (halve while every axis is even
-// and the coarse grid keeps at least 2 elements per axis, down to ~2k nodes).
+// and the coarse grid keeps at least 2 elements per axis, down to a grid that
+// is solved exactly).
+constexpr long long kDenseCoarseNodes = 768;
 int plan_levels(const Grid& g, int requested) {
   int nx = g.nx, ny = g.ny, nz = g.nz, lv = 1;
   const int maxlv = requested > 0 ? requested : 16;
   while (lv < maxlv) {
     if ((nx & 1) || (ny & 1) || (nz & 1) || nx < 4 || ny < 4 || nz < 4) break;
-    if (requested <= 0 && (long long)(nx + 1) * (ny + 1) * (nz + 1) <= 2500) break;
+    if (requested <= 0 && (long long)(nx + 1) * (ny + 1) * (nz + 1) <= kDenseCoarseNodes) break;
     nx >>= 1; ny >>= 1; nz >>= 1;
     ++lv;
   }
@@ -269,113 +271,38 @@ bool build_mg(Ctx& c, MG<T>& mg, const Grid& g0, const Mask& m0, const T* fac0, 
   return Lc.dinv && Lc.p && Lc.q && Lc.z && Lc.xa;
 }
 
-// Coarsest grids of at most this many free DOFs are solved exactly by one
-// dense matvec with the inverse of (K + sigma I) on their free DOFs (Cholesky
-// and inverse in FP64 on the host at setup, about n^3 flops, well under 0.1 s
-// at the limit); larger ones by the coarse PCG.  The count is of free DOFs:
-// the 8x4x4 coarsest grid of a 256x128x128 hierarchy has 675 DOFs, 600 of
-// them free once its x = 0 face is clamped.
-constexpr long long kDenseCoarse = 640;
+// Coarsest grids of at most kDenseCoarse DOFs are solved exactly, by the dense
+// inverse of (K + sigma I) on their free DOFs; the automatic level count
+// coarsens down to that where the grid allows it.  The inverse costs n^3/2 FP64
+// multiply-adds (about 10 ms at the limit, 0.6 ms at 600 DOFs), which 10 visits
+// of the one-CTA PCG on a grid of that size take.
+constexpr long long kDenseCoarse = 3 * kDenseCoarseNodes;
 
 template <typename T>
 void coarse_dense_setup(Ctx& c, MG<T>& mg, double sigma_c) {
   Lev<T>& V = mg.L.back();
   V.ainv = nullptr;
   const long long n = V.g.ndof();
-  if (n > 4 * kDenseCoarse || mg.ke.size() != 576) return;
-  const Grid& g = V.g;
-  std::vector<T> fac(g.nelem());
-  std::vector<uint8_t> mask;
-  cudaMemcpyAsync(fac.data(), V.fac, sizeof(T) * fac.size(), cudaMemcpyDeviceToHost, c.st);
-  if (V.m.node) {
-    mask.resize(g.nnode());
-    cudaMemcpyAsync(mask.data(), V.m.node, mask.size(), cudaMemcpyDeviceToHost, c.st);
-  }
-  if (cudaStreamSynchronize(c.st) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
-  // free DOFs: the device's fixed_bits (clamped faces, then the node mask)
-  const uint32_t F = V.m.faces;
-  std::vector<int> fidx(n, -1);
-  int nf = 0;
-  for (int k = 0; k < g.NZ; ++k)
-    for (int j = 0; j < g.NY; ++j)
-      for (int i = 0; i < g.NX; ++i) {
-        const long long nd = i + (long long)g.NX * (j + (long long)g.NY * k);
-        unsigned fx = (((F & 1u) && i == 0) || ((F & 2u) && i == g.NX - 1) || ((F & 4u) && j == 0) ||
-                       ((F & 8u) && j == g.NY - 1) || ((F & 16u) && k == 0) || ((F & 32u) && k == g.NZ - 1))
-                          ? 7u : 0u;
-        if (!mask.empty()) fx |= mask[nd];
-        for (int cc = 0; cc < 3; ++cc)
-          if (!((fx >> cc) & 1u)) fidx[3 * nd + cc] = nf++;
-      }
-  if (nf == 0 || nf > kDenseCoarse) return;
-  std::vector<double> A((size_t)nf * nf, 0.0);
-  for (int q = 0; q < nf; ++q) A[(size_t)q * nf + q] = sigma_c;
-  static const int ref_to_corner[8] = {0, 1, 3, 2, 4, 5, 7, 6};  // K0 node order (Mesh.jl:45-53) -> dx + 2dy + 4dz
-  long long dof[24];
-  for (int k = 0; k < g.nz; ++k)
-    for (int j = 0; j < g.ny; ++j)
-      for (int i = 0; i < g.nx; ++i) {
-        const double f = (double)fac[i + (long long)g.nx * (j + (long long)g.ny * k)];
-        for (int a = 0; a < 8; ++a) {
-          const int cc = ref_to_corner[a];
-          const long long nd = (i + (cc & 1)) + (long long)g.NX * ((j + ((cc >> 1) & 1)) + (long long)g.NY * (k + (cc >> 2)));
-          for (int d = 0; d < 3; ++d) dof[3 * a + d] = fidx[3 * nd + d];
-        }
-        for (int r = 0; r < 24; ++r) {
-          if (dof[r] < 0) continue;
-          for (int q = 0; q < 24; ++q)
-            if (dof[q] >= 0) A[(size_t)dof[r] * nf + dof[q]] += f * mg.ke[r + 24 * q];
-        }
-      }
-  // Cholesky A = L L^T (lower, in place); give up (coarse PCG) on a non-positive pivot
-  for (int jj = 0; jj < nf; ++jj) {
-    double d = A[(size_t)jj * nf + jj];
-    for (int m = 0; m < jj; ++m) d -= A[(size_t)jj * nf + m] * A[(size_t)jj * nf + m];
-    if (!(d > 0.0)) return;
-    const double ljj = std::sqrt(d);
-    A[(size_t)jj * nf + jj] = ljj;
-    for (int ii = jj + 1; ii < nf; ++ii) {
-      double v = A[(size_t)ii * nf + jj];
-      for (int m = 0; m < jj; ++m) v -= A[(size_t)ii * nf + m] * A[(size_t)jj * nf + m];
-      A[(size_t)ii * nf + jj] = v / ljj;
-    }
-  }
-  // inverse, column by column: L y = e_q, L^T x = y
-  std::vector<double> inv((size_t)nf * nf), y(nf);
-  for (int q = 0; q < nf; ++q) {
-    for (int ii = 0; ii < nf; ++ii) {
-      double v = ii == q ? 1.0 : 0.0;
-      for (int m = q; m < ii; ++m) v -= A[(size_t)ii * nf + m] * y[m];
-      y[ii] = ii < q ? 0.0 : v / A[(size_t)ii * nf + ii];
-    }
-    for (int ii = nf - 1; ii >= 0; --ii) {
-      double v = y[ii];
-      for (int m = ii + 1; m < nf; ++m) v -= A[(size_t)m * nf + ii] * y[m];
-      y[ii] = v / A[(size_t)ii * nf + ii];
-    }
-    for (int ii = 0; ii < nf; ++ii) inv[(size_t)ii * nf + q] = y[ii];
-  }
-  // embed (zero rows/columns at fixed DOFs); symmetric, so either order reads coalesced
-  std::vector<T> full((size_t)n * n, T(0));
-  for (long long a = 0; a < n; ++a) {
-    if (fidx[a] < 0) continue;
-    for (long long b = 0; b < n; ++b)
-      if (fidx[b] >= 0) full[(size_t)a * n + b] = (T)inv[(size_t)fidx[a] * nf + fidx[b]];
-  }
-  T* d = c.vec<T>(std::string(sizeof(T) == 8 ? "mgdense64" : "mgdense32"), (size_t)n * n);
-  if (!d) {
+  if (n > kDenseCoarse || mg.ke.size() != 576) return;
+  const size_t np = dense_padded(n);
+  double* A = c.vec<double>("mgdense_a", np * np);
+  double* panels = c.vec<double>("mgdense_p", 2 * np * 32 + 1024);
+  double* ke = c.vec<double>("mgdense_ke", 576);
+  int* flag = c.vec<int>("mgdense_flag", 1);
+  T* out = c.vec<T>(sizeof(T) == 8 ? "mgdense64" : "mgdense32", (size_t)n * dense_ld(n));
+  if (!A || !panels || !ke || !flag || !out) {  // the coarse PCG needs none of it
     c.err.clear();
     return;
   }
-  cudaMemcpyAsync(d, full.data(), sizeof(T) * full.size(), cudaMemcpyHostToDevice, c.st);
+  cudaMemcpyAsync(ke, mg.ke.data(), sizeof(double) * 576, cudaMemcpyHostToDevice, c.st);
+  c.launches += launch_dense_inverse<T>(V.g, V.m, V.fac, ke, sigma_c, A, panels, flag, out, c.st);
+  int bad = 0;
+  cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, c.st);
   if (cudaStreamSynchronize(c.st) != cudaSuccess) {
     cudaGetLastError();
     return;
   }
-  V.ainv = d;
+  if (!bad) V.ainv = out;  // a pivot that is not positive: the coarse PCG
 }
 
 template <typename T>
