@@ -755,6 +755,211 @@ __global__ void __launch_bounds__(1024) batch_coarse_pcg_smem_kernel(const Batch
   for (int i = tid; i < n3; i += nthr) gx[i] = sx[i];
 }
 
+// The same PCG where the grid has at most 1024 nodes and elements (every
+// automatic batch hierarchy): a thread keeps up to two nodes' x, r, p and D^-1 in
+// registers, so shared memory holds only p (read by the elements) and the
+// element products, both as (x, y) pairs plus z, with the butterflies in packed
+// FP32x2.  A node's elements past the grid point at a slot of zeros.  Four
+// barriers an iteration and no integer division inside the loop.  Bound by
+// instruction issue on its one SM: 12x6x6 to 14x7x7 grids, 30 iterations:
+// 65 us a launch against 91 to 105 us for the form above.
+constexpr int kRegMax = 1024, kRegThreads = 512;
+struct CoarseRegSmem {
+  float2 wxy[8][kRegMax + 1];
+  float wz[8][kRegMax + 1];
+  float2 pxy[kRegMax];
+  float pz[kRegMax];
+  float red[2][kRegThreads / 32];
+};
+__device__ __forceinline__ float2 f2add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 f2sub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+
+// h: corner values in, f K0 u out (corner order dx + 2dy + 4dz)
+__device__ __forceinline__ void element_product_packed(const ModalK<float>& K, float f, float2 (&hxy)[8], float (&hz)[8]) {
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int lo = 0; lo < 8; ++lo)
+      if (!((lo >> d) & 1)) {
+        const int hi = lo | (1 << d);
+        const float2 a = hxy[lo], b = hxy[hi];
+        hxy[lo] = f2add(a, b), hxy[hi] = f2sub(b, a);
+        const float az = hz[lo], bz = hz[hi];
+        hz[lo] = az + bz, hz[hi] = bz - az;
+      }
+  float2 wxy[8];
+  float wz[8];
+#pragma unroll
+  for (int mm = 0; mm < 8; ++mm) {
+    float w[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int qq = mm ^ (1 << c);
+      float t = 0.f;
+#pragma unroll
+      for (int c2 = 0; c2 < 3; ++c2)
+        if (modal_nz_mg(qq, c, c2)) {
+          const int m2 = qq ^ (1 << c2);
+          t = fmaf(K.B[qq][c][c2], c2 == 0 ? hxy[m2].x : (c2 == 1 ? hxy[m2].y : hz[m2]), t);
+        }
+      w[c] = t;
+    }
+    wxy[mm] = __fmul2_rn(make_float2(w[0], w[1]), make_float2(f, f));
+    wz[mm] = w[2] * f;
+  }
+#pragma unroll
+  for (int d = 2; d >= 0; --d)
+#pragma unroll
+    for (int lo = 0; lo < 8; ++lo)
+      if (!((lo >> d) & 1)) {
+        const int hi = lo | (1 << d);
+        const float2 a = wxy[lo], b = wxy[hi];
+        wxy[lo] = f2sub(a, b), wxy[hi] = f2add(a, b);
+        const float az = wz[lo], bz = wz[hi];
+        wz[lo] = az - bz, wz[hi] = az + bz;
+      }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) hxy[c] = wxy[c], hz[c] = wz[c];
+}
+
+__global__ void __launch_bounds__(kRegThreads, 1)
+    batch_coarse_pcg_reg_kernel(const BatchInst* in, const float* __restrict__ fac, const __grid_constant__ ModalK<float> K,
+                                const float* __restrict__ dinv, const float* __restrict__ b, float* xout, int iters,
+                                const PcgScalars* s) {
+  extern __shared__ __align__(16) unsigned char coarse_smem[];
+  CoarseRegSmem& S = *reinterpret_cast<CoarseRegSmem*>(coarse_smem);
+  const BatchInst& I = in[blockIdx.x];
+  if (batch_halted(s, I.id)) return;
+  const Grid g = I.g;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int ne = (int)g.nelem(), nn = (int)g.nnode(), nxy = g.NX * g.NY;
+  const float sigma = (float)I.sigma;
+  int phase = 0;
+  // one barrier: the other half of red is in use until the next sum's barrier
+  auto block_sum = [&](float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) S.red[phase][wid] = v;
+    __syncthreads();
+    v = S.red[phase][lane & (kRegThreads / 32 - 1)];
+#pragma unroll
+    for (int o = kRegThreads / 64; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    phase ^= 1;
+    return v;
+  };
+  int enode[2];
+  float ef[2];
+  unsigned short eo[2][8];  // the 8 elements around a node (kRegMax: none)
+  unsigned fx[2];
+  float x[2][3], r[2][3], p[2][3], di[2][3];
+  float part = 0.f;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int t = tid + u * kRegThreads;
+    enode[u] = 0;
+    ef[u] = 0.f;
+    if (t < ne) {
+      const int i = t % g.nx, q = t / g.nx;
+      enode[u] = i + g.NX * (q % g.ny + g.NY * (q / g.ny));
+      ef[u] = fac[I.eoff + t];
+    }
+    const int i = t % g.NX, q = t / g.NX, j = q % g.NY, k = q / g.NY;
+    fx[u] = t < nn ? fixed_bits(g, I.m, i, j, k, t) : 7u;
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+      const int ei = i - 1 + (o & 1), ej = j - 1 + ((o >> 1) & 1), ek = k - 1 + (o >> 2);
+      const bool ok = t < nn && ei >= 0 && ei < g.nx && ej >= 0 && ej < g.ny && ek >= 0 && ek < g.nz;
+      eo[u][o] = (unsigned short)(ok ? ei + g.nx * (ej + g.ny * ek) : kRegMax);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      x[u][c] = 0.f;
+      r[u][c] = t < nn ? b[I.off + 3 * t + c] : 0.f;
+      di[u][c] = t < nn ? dinv[I.off + 3 * t + c] : 0.f;
+      p[u][c] = di[u][c] * r[u][c];
+      part = fmaf(r[u][c], p[u][c], part);
+    }
+    if (t < nn) S.pxy[t] = make_float2(p[u][0], p[u][1]), S.pz[t] = p[u][2];
+  }
+  if (tid < 8) S.wxy[tid][kRegMax] = make_float2(0.f, 0.f), S.wz[tid][kRegMax] = 0.f;
+  float rz = block_sum(part);  // its barrier also publishes p and the zero slot
+  for (int it = 0; it < iters; ++it) {
+#pragma unroll 1
+    for (int u = 0; u < 2; ++u) {
+      const int e = tid + u * kRegThreads;
+      if (e < ne) {
+        const int n0 = u ? enode[1] : enode[0];
+        float2 hxy[8];
+        float hz[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const int nd = n0 + (c & 1) + ((c >> 1) & 1 ? g.NX : 0) + (c >> 2 ? nxy : 0);
+          hxy[c] = S.pxy[nd];
+          hz[c] = S.pz[nd];
+        }
+        element_product_packed(K, u ? ef[1] : ef[0], hxy, hz);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) S.wxy[c][e] = hxy[c], S.wz[c][e] = hz[c];
+      }
+    }
+    __syncthreads();
+    float q[2][3];
+    part = 0.f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (tid + u * kRegThreads >= nn) {
+        q[u][0] = q[u][1] = q[u][2] = 0.f;
+        continue;
+      }
+      float2 sxy = make_float2(0.f, 0.f);
+      float sz = 0.f;
+#pragma unroll
+      for (int o = 0; o < 8; ++o) {
+        sxy = f2add(sxy, S.wxy[7 - o][eo[u][o]]);
+        sz += S.wz[7 - o][eo[u][o]];
+      }
+      const float sv[3] = {sxy.x, sxy.y, sz};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        q[u][c] = ((fx[u] >> c) & 1u) ? 0.f : fmaf(sigma, p[u][c], sv[c]);
+        part = fmaf(p[u][c], q[u][c], part);
+      }
+    }
+    const float pAp = block_sum(part);
+    if (!(pAp > 0.f)) break;  // converged to rounding or no curvature left
+    const float alpha = rz / pAp;
+    part = 0.f;
+    float z[2][3];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        x[u][c] = fmaf(alpha, p[u][c], x[u][c]);
+        r[u][c] = fmaf(-alpha, q[u][c], r[u][c]);
+        z[u][c] = di[u][c] * r[u][c];
+        part = fmaf(r[u][c], z[u][c], part);
+      }
+    const float rz_new = block_sum(part);
+    const float beta = rz != 0.f ? rz_new / rz : 0.f;
+    rz = rz_new;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = tid + u * kRegThreads;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) p[u][c] = fmaf(beta, p[u][c], z[u][c]);
+      if (t < nn) S.pxy[t] = make_float2(p[u][0], p[u][1]), S.pz[t] = p[u][2];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int t = tid + u * kRegThreads;
+    if (t < nn)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) xout[I.off + 3 * t + c] = x[u][c];
+  }
+}
+
 // Shared memory a smem form needs for the largest coarsest grid of a launch
 // (0: too large for that form).
 template <typename T>
@@ -767,6 +972,18 @@ template <typename T>
 void launch_batch_coarse_pcg(const BatchInst* in, int ninst, const T* fac, const ModalK<T>& K, const T* dinv,
                              const T* b, T* x, T* r, T* z, T* p, T* q, T* w, int iters, const PcgScalars* s,
                              cudaStream_t st, long long max_ndof, long long max_nelem) {
+  if constexpr (sizeof(T) == 4) {
+    if (max_ndof <= 3 * kRegMax && max_nelem <= kRegMax) {
+      static bool attr_reg = false;
+      if (!attr_reg) {
+        cudaFuncSetAttribute(batch_coarse_pcg_reg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(CoarseRegSmem));
+        attr_reg = true;
+      }
+      batch_coarse_pcg_reg_kernel<<<ninst, kRegThreads, sizeof(CoarseRegSmem), st>>>(in, fac, K, dinv, b, x, iters, s);
+      return;
+    }
+  }
   const size_t smem_w = batch_coarse_smem_bytes<T>(max_ndof, max_nelem, true);
   const size_t smem_c = batch_coarse_smem_bytes<T>(max_ndof, max_nelem, false);
   static bool attr = false;
