@@ -17,6 +17,7 @@ enum OpMode {
   OP_CHEB2 = 5,       // y = x + c1 (x - xin) + c2 D^-1 (b - Ax)   (xin null: 0; y may alias xin)
   OP_JACOBI_DOT = 6,  // OP_JACOBI, sum b.y (r.z of the V-cycle's last step)
   OP_CHEB2_DOT = 7,   // OP_CHEB2, sum b.y
+  OP_APPLY_MASK = 8,  // y = A (x with its fixed DOFs taken as zero); one column, not in batches
 };
 
 template <typename T>
@@ -44,6 +45,8 @@ struct OpArgs {
 
 template <typename T>
 void launch_op(int mode, const OpArgs<T>& a, cudaStream_t st);
+// Whether FP32 launches use the TMA-staged form (which has no OP_APPLY_MASK).
+bool op_staged_form();
 // Whether a staged FP32 operator launch gave up a bounded wait since the last
 // call (reads and clears the device word; synchronizes st).
 bool op_take_wait_error(cudaStream_t st);
@@ -66,6 +69,8 @@ void launch_copy(T* dst, const T* src, long long n, cudaStream_t st);
 // dst = src with fixed DOFs zeroed (expand/contract semantics)
 template <typename TD, typename TS>
 void launch_mask_copy(const Grid& g, const Mask& m, TD* dst, const TS* src, cudaStream_t st);
+// Per-node bits (bit c: component c fixed) from one byte per DOF
+void launch_node_bits(const uint8_t* fixed_dof, uint8_t* bits, long long nnode, cudaStream_t st);
 // Jacobi inverse diagonal dinv = 1/(dd*fsum + sigma) (0 at fixed DOFs) and
 // the raw diagonal (dd*fsum, 0 at fixed DOFs).
 template <typename T>

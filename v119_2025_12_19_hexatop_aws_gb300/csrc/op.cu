@@ -345,8 +345,12 @@ __device__ __forceinline__ void op_item(const A& a, int tx, int ty, int chunk,
                                         T (&xch)[2][TYW][32][4],
                                         double& acc0, long long co) {
   // the _DOT forms of the smoothing steps also sum b.y
-  constexpr int BM = MODE == OP_JACOBI_DOT ? OP_JACOBI : (MODE == OP_CHEB2_DOT ? OP_CHEB2 : MODE);
+  constexpr int BM = MODE == OP_JACOBI_DOT ? OP_JACOBI
+                     : MODE == OP_CHEB2_DOT ? OP_CHEB2
+                     : MODE == OP_APPLY_MASK ? OP_APPLY
+                                             : MODE;
   constexpr bool DOTB = MODE == OP_JACOBI_DOT || MODE == OP_CHEB2_DOT;
+  constexpr bool MASKX = MODE == OP_APPLY_MASK;  // x may hold anything at fixed DOFs
   constexpr int NX_OWN = 31, NY_OWN = TYW - 1;
   constexpr bool NEED_F = (BM == OP_JACOBI || BM == OP_CHEB2);
   static_assert(TYW <= 16, "pairwise barriers use the named barriers 1..TYW-1");
@@ -379,14 +383,51 @@ __device__ __forceinline__ void op_item(const A& a, int tx, int ty, int chunk,
   auto facload = [&](int k) -> T {
     return (colv && k >= 0 && k < g.nz) ? ldx(fac + ecol + eplane * k) : T(0);
   };
+  // MASKX: the corners' fixed bits (3 per corner): x and y faces per column,
+  // the z faces and the optional node mask per layer.  Applied where the values
+  // are used, so that the loads stay one layer ahead; a warp whose columns
+  // touch no fixed DOF skips the selects.
+  unsigned cfix = 0;
+  if (MASKX) {
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) {
+      const int i = ie + (cc & 1), j = je + (cc >> 1);
+      if (((F & 1u) && i <= 0) || ((F & 2u) && i >= g.NX - 1) || ((F & 4u) && j <= 0) || ((F & 8u) && j >= g.NY - 1))
+        cfix |= 7u << (3 * cc);
+    }
+  }
+  auto load_bits = [&](int kk) -> unsigned {
+    if (!MASKX) return 0u;
+    unsigned m = cfix;
+    if (((F & 16u) && kk <= 0) || ((F & 32u) && kk >= g.NZ - 1)) m = 0xfffu;
+    if (a.m.node) {
+      const IX L = (IX)(nplane * (IX)min(max(kk, 0), g.NZ - 1));
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) {
+        const int i = min(max(ie + (cc & 1), 0), g.NX - 1), j = min(max(je + (cc >> 1), 0), g.NY - 1);
+        m |= (unsigned)__ldg(a.m.node + (L + (IX)i + (IX)g.NX * j)) << (3 * cc);
+      }
+    }
+    return m;
+  };
+  auto drop_fixed = [&](T (&v)[4][3], unsigned m) {
+    if (MASKX && m) {
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[cc][c] = ((m >> (3 * cc + c)) & 1u) ? T(0) : v[cc][c];
+    }
+  };
   T Lm[4][3], carry[4][3], xown[3];
   T fprev;
   {
     T raw[4][3];
     load_corners<T, IX, INTERIOR>(g, ca, x, k0 - 1, raw);
+    drop_fixed(raw, load_bits(k0 - 1));
     T Lprev[4][3];
     xy_forward<T>(raw, Lprev);
     load_corners<T, IX, INTERIOR>(g, ca, x, k0, raw);
+    drop_fixed(raw, load_bits(k0));
 #pragma unroll
     for (int c = 0; c < 3; ++c) xown[c] = raw[3][c];
     xy_forward<T>(raw, Lm);
@@ -417,6 +458,7 @@ __device__ __forceinline__ void op_item(const A& a, int tx, int ty, int chunk,
   T accT = T(0);
   T nraw[4][3];
   load_corners<T, IX, INTERIOR>(g, ca, x, k0 + 1, nraw);
+  unsigned nbits = load_bits(k0 + 1);
   T fnext = facload(k0);
 
   // three layers per unrolled step for the Chebyshev forms, two for the rest
@@ -429,12 +471,14 @@ __device__ __forceinline__ void op_item(const A& a, int tx, int ty, int chunk,
     for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
       for (int c = 0; c < 3; ++c) raw[cc][c] = nraw[cc][c];
+    drop_fixed(raw, nbits);
     const T f = fnext;
     T bk[3], pk3[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) bk[c] = bnext[c], pk3[c] = pnext[c];
     if (k + 1 < k1) {  // prefetch the next layer
       load_corners<T, IX, INTERIOR>(g, ca, x, k + 2, nraw);
+      nbits = load_bits(k + 2);
       fnext = facload(k + 1);
       if (NEED_B || NEED_P) load_bp(k + 1);
     }
@@ -961,6 +1005,7 @@ template <typename T>
 static int resident_ctas(int mode) {
   switch (mode) {
     case OP_APPLY: return op_resident_ctas<T, OP_APPLY>();
+    case OP_APPLY_MASK: return op_resident_ctas<T, OP_APPLY_MASK>();
     case OP_APPLY_DOT: return op_resident_ctas<T, OP_APPLY_DOT>();
     case OP_RESID: return op_resident_ctas<T, OP_RESID>();
     case OP_RESID_NORM: return op_resident_ctas<T, OP_RESID_NORM>();
@@ -1046,7 +1091,10 @@ static int tma_resident_ctas() {
   return cached;
 }
 
+bool op_staged_form() { return op_form() == 1; }
+
 bool op_take_wait_error(cudaStream_t st) {
+  if (!op_staged_form()) return false;  // only that form waits
   int h = 0;
   if (cudaMemcpyFromSymbolAsync(&h, g_op_wait_err, sizeof(int), 0, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess) {
@@ -1132,6 +1180,7 @@ void launch_op(int mode, const OpArgs<T>& a0, cudaStream_t st) {
     HEXA_OP_CASE(OP_CHEB2)
     HEXA_OP_CASE(OP_JACOBI_DOT)
     HEXA_OP_CASE(OP_CHEB2_DOT)
+    HEXA_OP_CASE(OP_APPLY_MASK)
     default: break;
   }
 #undef HEXA_OP_CASE

@@ -34,6 +34,10 @@ struct Ctx {
   };
   std::map<std::string, Tuned> tuned;
   double* hscal = nullptr;   // pinned host mirror of dscal
+  // modal blocks of the last element geometry (0.1 ms of host quadrature)
+  double modal_key[4] = {0.0, 0.0, 0.0, 0.0};  // dx, dy, dz, nu
+  ModalK<double> modal;
+  bool modal_ok = false;
 
   void* get(const std::string& name, size_t bytes);
   template <typename T>

@@ -110,6 +110,15 @@ void launch_mask_copy(const Grid& g, const Mask& m, TD* dst, const TS* src, cuda
   mask_copy_kernel<TD, TS><<<vec_blocks(g.nnode()), 256, 0, st>>>(g, m, dst, src);
 }
 
+// A warp's 32 nodes are 96 mask bytes: three coalesced byte loads per thread.
+__global__ void node_bits_kernel(const uint8_t* __restrict__ fixed, uint8_t* __restrict__ bits, long long nn) {
+  for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nn; n += (long long)gridDim.x * blockDim.x)
+    bits[n] = (uint8_t)((fixed[3 * n] ? 1 : 0) | (fixed[3 * n + 1] ? 2 : 0) | (fixed[3 * n + 2] ? 4 : 0));
+}
+void launch_node_bits(const uint8_t* fixed_dof, uint8_t* bits, long long nnode, cudaStream_t st) {
+  node_bits_kernel<<<vec_blocks(nnode), 256, 0, st>>>(fixed_dof, bits, nnode);
+}
+
 // Sum of the factors of the (up to) 8 elements around node (i,j,k).
 template <typename T>
 __device__ __forceinline__ T node_factor_sum(const Grid& g, const T* __restrict__ fac, int i, int j,
