@@ -814,12 +814,16 @@ int hexa_update_density(hexa_ctx* h, const hexa_grid* g, float* density, const f
   const float* od = stage_in<float>(c, original_density, ne, "ud_orig");
   const uint8_t* pd = protected_mask ? stage_in<uint8_t>(c, protected_mask, ne, "ud_prot") : nullptr;
   const float* dd = stage_in<float>(c, (const float*)density, ne, "ud_rho");  // the user's array is written last
-  float* prop = c.vec<float>("ud_prop", ne);
+  st.R_length = density_filter_radius(*p, (float)g->dx, (float)g->dy, (float)g->dz);
+  st.R_effective = st.R_length / 2.5f;
+  const bool filtered = (double)st.R_effective > 1e-4;
+  float* prop = filtered ? c.vec<float>("ud_prop", ne) : nullptr;
   float* work = c.vec<float>("ud_new", ne);
   UpdateState* s = c.vec<UpdateState>("ud_state", 1);
   double* part = c.vec<double>("ud_part", update_partials_doubles());
   unsigned long long* hist = c.vec<unsigned long long>("ud_hist", update_hist_bins());
-  if (!l1d || !od || (protected_mask && !pd) || !dd || !prop || !work || !s || !part || !hist)
+  unsigned* tie = c.vec<unsigned>("ud_tie", update_ties());
+  if (!l1d || !od || (protected_mask && !pd) || !dd || (filtered && !prop) || !work || !s || !part || !hist || !tie)
     return set_err(h, HEXA_ERR_NOMEM, c.err.empty() ? "density update: out of device memory" : c.err);
   static_assert(sizeof(UpdateState) <= 16 * sizeof(double), "UpdateState exceeds its host landing slots");
   UpdateState* hs = reinterpret_cast<UpdateState*>(c.hscal + 48);
@@ -828,19 +832,32 @@ int hexa_update_density(hexa_ctx* h, const hexa_grid* g, float* density, const f
     return cudaStreamSynchronize(c.st) == cudaSuccess && c.cuda_ok("update_density");
   };
   cudaMemsetAsync(s, 0, sizeof(UpdateState), c.st);
-  launch_propose(ne, l1d, pd, od, p->l1_stress_allowable, p->E, p->min_density, prop, s, c.st);
-  c.launches++;
-  if (!fetch()) return set_err(h, HEXA_ERR_CUDA, c.err);
-  if (hs->nan_stress) {  // TopOpt.jl:230-236: no update, zero statistics
+  // the result goes straight into a device density (the finishing pass writes
+  // nothing after a NaN), else into the scratch and to the host
+  const bool on_device = is_device_ptr(density);
+  float* res = on_device ? density : work;
+  st.current_threshold = density_cull_threshold(*p);
+  auto cull = [&](bool fused, const float* src) {
+    c.launches += launch_update_cull(fused, ne, dd, src, pd, od, p->l1_stress_allowable, p->E, p->min_density,
+                                     p->max_density, st.current_threshold, p->max_culling_ratio,
+                                     p->hard_update ? 1 : 0, work, res, part, hist, tie, s, c.st);
+    return fetch();
+  };
+  auto nan_stress = [&]() {  // TopOpt.jl:230-236: no update, zero statistics
+    std::memset(&st, 0, sizeof(st));
     st.status = 1;
     if (stats) *stats = st;
     return HEXA_OK;
-  }
-  st.R_length = density_filter_radius(*p, (float)g->dx, (float)g->dy, (float)g->dz);
-  st.R_effective = st.R_length / 2.5f;
-  st.current_threshold = density_cull_threshold(*p);
-  const float* src = prop;
-  if ((double)st.R_effective > 1e-4) {
+  };
+  if (!filtered) {
+    if (!cull(true, l1d)) return set_err(h, HEXA_ERR_CUDA, c.err);
+    if (hs->nan_stress) return nan_stress();
+  } else {
+    launch_propose(ne, l1d, pd, od, p->l1_stress_allowable, p->E, p->min_density, prop, s, c.st);
+    c.launches++;
+    if (!fetch()) return set_err(h, HEXA_ERR_CUDA, c.err);
+    if (hs->nan_stress) return nan_stress();
+    const float* src = prop;
     st.filter_used = 1;
     double Ke[64], Me[64];
     if (scalar_matrices(g->dx, g->dy, g->dz, 1, Ke, Me) != 0) return set_err(h, HEXA_ERR_ARG, "invalid element size");
@@ -862,23 +879,22 @@ int hexa_update_density(hexa_ctx* h, const hexa_grid* g, float* density, const f
     st.filter_time = fs.solve_ms / 1e3;
     st.filter_iters = fs.iterations;
     st.filter_res = fs.relres;
-  }
-  c.launches += launch_update_cull(ne, dd, src, pd, od, p->min_density, p->max_density, st.current_threshold,
-                                   p->max_culling_ratio, p->hard_update ? 1 : 0, work, part, hist, s, c.st);
-  if (!fetch()) return set_err(h, HEXA_ERR_CUDA, c.err);
-  if (hs->nan_filtered && src != prop) {  // TopOpt.jl:360-363: the unfiltered proposal instead
-    st.filter_nan_fallback = 1;
-    c.launches += launch_update_cull(ne, dd, prop, pd, od, p->min_density, p->max_density, st.current_threshold,
-                                     p->max_culling_ratio, p->hard_update ? 1 : 0, work, part, hist, s, c.st);
-    if (!fetch()) return set_err(h, HEXA_ERR_CUDA, c.err);
+    if (!cull(false, src)) return set_err(h, HEXA_ERR_CUDA, c.err);
+    if (hs->nan_filtered) {
+      st.filter_nan_fallback = src != prop ? 1 : 0;  // TopOpt.jl:360-363: the unfiltered proposal instead
+      cudaMemsetAsync(&s->nan_filtered, 0, sizeof(int), c.st);
+      if (!cull(true, l1d)) return set_err(h, HEXA_ERR_CUDA, c.err);
+    }
   }
   st.mean_change = hs->mean_change;
   st.active_count = (int64_t)hs->active;
   st.candidates = (int64_t)hs->candidates;
   st.culled = (int64_t)hs->culled;
-  cudaMemcpyAsync(density, work, ne * sizeof(float),
-                  is_device_ptr(density) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, c.st);
-  if (cudaStreamSynchronize(c.st) != cudaSuccess || !c.cuda_ok("update_density")) return set_err(h, HEXA_ERR_CUDA, c.err);
+  if (!on_device) {
+    cudaMemcpyAsync(density, work, ne * sizeof(float), cudaMemcpyDeviceToHost, c.st);
+    if (cudaStreamSynchronize(c.st) != cudaSuccess || !c.cuda_ok("update_density"))
+      return set_err(h, HEXA_ERR_CUDA, c.err);
+  }
   if (stats) *stats = st;
   return HEXA_OK;
 }

@@ -212,18 +212,25 @@ void launch_remap_nodal(int onx, int ony, int onz, int nnx, int nny, int nnz, co
 
 // ---- density update between solves (update.cu) -----------------------------
 struct UpdateState {
-  int nan_stress, nan_filtered, mode, pad;  // mode: 0 cull none, 1 every candidate, 2 the `allowed` smallest
+  int nan_stress, nan_filtered, mode, done;  // mode: 0 cull none, 1 every candidate, 2 the `allowed` smallest
   double change;                            // sum of |min(raw, max) - old| over unprotected elements
   unsigned long long active_updated;        // unprotected raw > min_density (the mean's divisor)
   unsigned long long active, candidates, allowed, culled;
   unsigned long long prefix, remaining;     // radix select: key of the last culled candidate
-  float mean_change, pad2;
+  unsigned long long ties;                  // candidates that share the digits picked so far
+  float mean_change;
+  unsigned ntie, ticket, pad;
 };
 void launch_propose(long long n, const float* l1, const uint8_t* prot, const float* orig, float allow, float E,
                     float min_d, float* prop, UpdateState* s, cudaStream_t st);
-int launch_update_cull(long long n, const float* old, const float* src, const uint8_t* prot, const float* orig,
-                       float min_d, float max_d, float thr, float ratio, int hard, float* out, double* part,
-                       unsigned long long* hist, UpdateState* s, cudaStream_t st);
+// fused: src = the stress norms, the proposal is formed in the pass; else src =
+// the (filtered) proposal.  work: n floats of scratch; res: the result (left
+// alone after a NaN); tie: update_ties() indices.
+int launch_update_cull(bool fused, long long n, const float* old, const float* src, const uint8_t* prot,
+                       const float* orig, float allow, float E, float min_d, float max_d, float thr, float ratio,
+                       int hard, float* work, float* res, double* part, unsigned long long* hist, unsigned* tie,
+                       UpdateState* s, cudaStream_t st);
+int update_ties();
 size_t update_partials_doubles();
 int update_hist_bins();
 
