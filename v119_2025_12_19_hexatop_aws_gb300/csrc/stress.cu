@@ -51,100 +51,131 @@ __device__ __forceinline__ void jacobi_rotate(float& spp, float& sqq, float& spq
   }
 }
 
+// A thread marches kStressZ elements of its column in z: the four nodes between
+// two elements are read and rounded once (conversions from FP64 run at the FP64
+// pipe's 2 per clock and SM), and the x and y parts of the Jacobian are formed
+// once.  Bound by instruction issue: the rotations' divisions and square roots,
+// then the index arithmetic, whose 64-bit divisions per element are gone.
+// 256x128x128 with the Voigt stress: 203 us (issue slots 74 % busy), 242 at one element per
+// thread; every operation on the values is the same, and so are the results.
+constexpr int kStressZ = 8;
 template <typename TU>
-__global__ void stress_kernel(Grid g, const TU* __restrict__ u, const float* __restrict__ density, float E, float nu,
-                              float dx, float dy, float dz, int save_voigt, float* __restrict__ principal,
-                              float* __restrict__ vonmises, float* __restrict__ voigt, float* __restrict__ l1,
-                              float* __restrict__ dmax, float* __restrict__ dmin) {
-  const long long ne = g.nelem();
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < ne;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % g.nx);
-    const long long t0 = e / g.nx;
-    const int j = (int)(t0 % g.ny), k = (int)(t0 / g.ny);
-    const float dens = density[e];
-    if (dens < 1.0e-6f) {
-#pragma unroll
-      for (int q = 0; q < 3; ++q) principal[3 * e + q] = 0.f, dmax[3 * e + q] = 0.f, dmin[3 * e + q] = 0.f;
-      vonmises[e] = 0.f;
-      l1[e] = 0.f;
-      if (save_voigt)
-#pragma unroll
-        for (int q = 0; q < 6; ++q) voigt[6 * e + q] = 0.f;
-      continue;
-    }
-    const float Eloc = E * dens;
+__global__ void __launch_bounds__(128) stress_kernel(Grid g, const TU* __restrict__ u, const float* __restrict__ density,
+                                                     float E, float nu, float dx, float dy, float dz, int save_voigt,
+                                                     float* __restrict__ principal, float* __restrict__ vonmises,
+                                                     float* __restrict__ voigt, float* __restrict__ l1,
+                                                     float* __restrict__ dmax, float* __restrict__ dmin) {
+  const int nbx = (g.nx + 31) / 32, nby = (g.ny + 3) / 4, nzc = (g.nz + kStressZ - 1) / kStressZ;
+  const long long items = (long long)nbx * nby * nzc;
+  for (long long item = blockIdx.x; item < items; item += gridDim.x) {
+    const int t = (int)(item / nbx), i = (int)(item - (long long)t * nbx) * 32 + threadIdx.x;
+    const int j = (t % nby) * 4 + threadIdx.y, k0 = t / nby * kStressZ, k1 = min(k0 + kStressZ, g.nz);
+    if (i >= g.nx || j >= g.ny) continue;
     // node a of the element in the reference's order n1..n8 (Mesh.jl:45-53)
     constexpr int DI[8] = {0, 1, 1, 0, 0, 1, 1, 0}, DJ[8] = {0, 0, 1, 1, 0, 0, 1, 1}, DK[8] = {0, 0, 0, 0, 1, 1, 1, 1};
-    float j11 = 0.f, j12 = 0.f, j13 = 0.f, j21 = 0.f, j22 = 0.f, j23 = 0.f, j31 = 0.f, j32 = 0.f, j33 = 0.f;
+    const long long col = (long long)i + (long long)g.NX * j, nplane = (long long)g.NX * g.NY;
+    float un[8][3];  // corner displacements; the lower four come from the element below
+    auto load_layer = [&](int k, int a0) {
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const float x = (float)(i + DI[a]) * dx, y = (float)(j + DJ[a]) * dy, z = (float)(k + DK[a]) * dz;
-      const float nxi = DI[a] ? 0.125f : -0.125f, net = DJ[a] ? 0.125f : -0.125f, nze = DK[a] ? 0.125f : -0.125f;
-      j11 += nxi * x; j12 += nxi * y; j13 += nxi * z;
-      j21 += net * x; j22 += net * y; j23 += net * z;
-      j31 += nze * x; j32 += nze * y; j33 += nze * z;
-    }
-    float det = j11 * (j22 * j33 - j23 * j32) - j12 * (j21 * j33 - j23 * j31) + j13 * (j21 * j32 - j22 * j31);
-    if (det <= 1.0e-12f) det = 1.0f;
-    const float id = 1.0f / det;
-    const float a11 = (j22 * j33 - j23 * j32) * id, a12 = -(j12 * j33 - j13 * j32) * id, a13 = (j12 * j23 - j13 * j22) * id;
-    const float a21 = -(j21 * j33 - j23 * j31) * id, a22 = (j11 * j33 - j13 * j31) * id, a23 = -(j11 * j23 - j13 * j21) * id;
-    const float a31 = (j21 * j32 - j22 * j31) * id, a32 = -(j11 * j32 - j12 * j31) * id, a33 = (j11 * j22 - j12 * j21) * id;
-    float exx = 0.f, eyy = 0.f, ezz = 0.f, gxy = 0.f, gyz = 0.f, gxz = 0.f;
+      for (int a = 0; a < 4; ++a) {
+        const TU* p = u + 3 * (col + DI[a] + (long long)g.NX * DJ[a] + nplane * k);
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const long long n = (long long)(i + DI[a]) + (long long)g.NX * ((long long)(j + DJ[a]) + (long long)g.NY * (k + DK[a]));
-      const float ux = (float)u[3 * n], uy = (float)u[3 * n + 1], uz = (float)u[3 * n + 2];
-      const float nxi = DI[a] ? 0.125f : -0.125f, net = DJ[a] ? 0.125f : -0.125f, nze = DK[a] ? 0.125f : -0.125f;
-      const float ddx = nxi * a11 + net * a21 + nze * a31;
-      const float ddy = nxi * a12 + net * a22 + nze * a32;
-      const float ddz = nxi * a13 + net * a23 + nze * a33;
-      exx += ddx * ux;
-      eyy += ddy * uy;
-      ezz += ddz * uz;
-      gxy += ddy * ux + ddx * uy;
-      gyz += ddz * uy + ddy * uz;
-      gxz += ddz * ux + ddx * uz;
-    }
-    const float fact = Eloc / ((1.0f + nu) * (1.0f - 2.0f * nu));
-    const float c1 = (1.0f - nu) * fact, c2 = nu * fact, c3 = (0.5f - nu) * fact;
-    const float sxx = c1 * exx + c2 * eyy + c2 * ezz;
-    const float syy = c2 * exx + c1 * eyy + c2 * ezz;
-    const float szz = c2 * exx + c2 * eyy + c1 * ezz;
-    const float sxy = c3 * gxy, syz = c3 * gyz, sxz = c3 * gxz;
-    if (save_voigt) {
-      voigt[6 * e] = sxx, voigt[6 * e + 1] = syy, voigt[6 * e + 2] = szz;
-      voigt[6 * e + 3] = sxy, voigt[6 * e + 4] = syz, voigt[6 * e + 5] = sxz;
-    }
-    const float vm2 = 0.5f * ((sxx - syy) * (sxx - syy) + (syy - szz) * (syy - szz) + (szz - sxx) * (szz - sxx)) +
-                      3.0f * (sxy * sxy + syz * syz + sxz * sxz);
-    vonmises[e] = sqrtf(fmaxf(0.0f, vm2));
-    // eigenpairs: cyclic Jacobi, at most 12 sweeps of the (1,2), (1,3), (2,3) rotations
-    float s11 = sxx, s22 = syy, s33 = szz, s12 = sxy, s23 = syz, s13 = sxz;
-    float v[3][3] = {{1.f, 0.f, 0.f}, {0.f, 1.f, 0.f}, {0.f, 0.f, 1.f}};
-    for (int it = 0; it < 12; ++it) {
-      if (fmaxf(fabsf(s12), fmaxf(fabsf(s23), fabsf(s13))) < 1.0e-9f) break;
-      jacobi_rotate(s11, s22, s12, s13, s23, v, 0, 1);
-      jacobi_rotate(s11, s33, s13, s12, s23, v, 0, 2);
-      jacobi_rotate(s22, s33, s23, s12, s13, v, 1, 2);
-    }
-    // descending order, columns of v swapped with their eigenvalues
-    auto swapcol = [&](int p, int q) {
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        const float t = v[r][p];
-        v[r][p] = v[r][q];
-        v[r][q] = t;
+        for (int c = 0; c < 3; ++c) un[a0 + a][c] = (float)p[c];
       }
     };
-    if (s11 < s22) { const float t = s11; s11 = s22; s22 = t; swapcol(0, 1); }
-    if (s22 < s33) { const float t = s22; s22 = s33; s33 = t; swapcol(1, 2); }
-    if (s11 < s22) { const float t = s11; s11 = s22; s22 = t; swapcol(0, 1); }
-    principal[3 * e] = s11, principal[3 * e + 1] = s22, principal[3 * e + 2] = s33;
+    load_layer(k0, 0);
+    for (int k = k0; k < k1; ++k) {
+      const long long e = (long long)i + (long long)g.nx * (j + (long long)g.ny * k);
+      load_layer(k + 1, 4);
+      const float dens = density[e];
+      if (dens < 1.0e-6f) {
 #pragma unroll
-    for (int r = 0; r < 3; ++r) dmax[3 * e + r] = v[r][0], dmin[3 * e + r] = v[r][2];
-    l1[e] = fabsf(s11) + fabsf(s22) + fabsf(s33);
+        for (int q = 0; q < 3; ++q) principal[3 * e + q] = 0.f, dmax[3 * e + q] = 0.f, dmin[3 * e + q] = 0.f;
+        vonmises[e] = 0.f;
+        l1[e] = 0.f;
+        if (save_voigt)
+#pragma unroll
+          for (int q = 0; q < 6; ++q) voigt[6 * e + q] = 0.f;
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) un[a][c] = un[a + 4][c];
+        continue;
+      }
+      const float Eloc = E * dens;
+      float j11 = 0.f, j12 = 0.f, j13 = 0.f, j21 = 0.f, j22 = 0.f, j23 = 0.f, j31 = 0.f, j32 = 0.f, j33 = 0.f;
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        const float x = (float)(i + DI[a]) * dx, y = (float)(j + DJ[a]) * dy, z = (float)(k + DK[a]) * dz;
+        const float nxi = DI[a] ? 0.125f : -0.125f, net = DJ[a] ? 0.125f : -0.125f, nze = DK[a] ? 0.125f : -0.125f;
+        j11 += nxi * x; j12 += nxi * y; j13 += nxi * z;
+        j21 += net * x; j22 += net * y; j23 += net * z;
+        j31 += nze * x; j32 += nze * y; j33 += nze * z;
+      }
+      float det = j11 * (j22 * j33 - j23 * j32) - j12 * (j21 * j33 - j23 * j31) + j13 * (j21 * j32 - j22 * j31);
+      if (det <= 1.0e-12f) det = 1.0f;
+      const float id = 1.0f / det;
+      const float a11 = (j22 * j33 - j23 * j32) * id, a12 = -(j12 * j33 - j13 * j32) * id, a13 = (j12 * j23 - j13 * j22) * id;
+      const float a21 = -(j21 * j33 - j23 * j31) * id, a22 = (j11 * j33 - j13 * j31) * id, a23 = -(j11 * j23 - j13 * j21) * id;
+      const float a31 = (j21 * j32 - j22 * j31) * id, a32 = -(j11 * j32 - j12 * j31) * id, a33 = (j11 * j22 - j12 * j21) * id;
+      float exx = 0.f, eyy = 0.f, ezz = 0.f, gxy = 0.f, gyz = 0.f, gxz = 0.f;
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        const float ux = un[a][0], uy = un[a][1], uz = un[a][2];
+        const float nxi = DI[a] ? 0.125f : -0.125f, net = DJ[a] ? 0.125f : -0.125f, nze = DK[a] ? 0.125f : -0.125f;
+        const float ddx = nxi * a11 + net * a21 + nze * a31;
+        const float ddy = nxi * a12 + net * a22 + nze * a32;
+        const float ddz = nxi * a13 + net * a23 + nze * a33;
+        exx += ddx * ux;
+        eyy += ddy * uy;
+        ezz += ddz * uz;
+        gxy += ddy * ux + ddx * uy;
+        gyz += ddz * uy + ddy * uz;
+        gxz += ddz * ux + ddx * uz;
+      }
+      const float fact = Eloc / ((1.0f + nu) * (1.0f - 2.0f * nu));
+      const float c1 = (1.0f - nu) * fact, c2 = nu * fact, c3 = (0.5f - nu) * fact;
+      const float sxx = c1 * exx + c2 * eyy + c2 * ezz;
+      const float syy = c2 * exx + c1 * eyy + c2 * ezz;
+      const float szz = c2 * exx + c2 * eyy + c1 * ezz;
+      const float sxy = c3 * gxy, syz = c3 * gyz, sxz = c3 * gxz;
+      if (save_voigt) {
+        voigt[6 * e] = sxx, voigt[6 * e + 1] = syy, voigt[6 * e + 2] = szz;
+        voigt[6 * e + 3] = sxy, voigt[6 * e + 4] = syz, voigt[6 * e + 5] = sxz;
+      }
+      const float vm2 = 0.5f * ((sxx - syy) * (sxx - syy) + (syy - szz) * (syy - szz) + (szz - sxx) * (szz - sxx)) +
+                        3.0f * (sxy * sxy + syz * syz + sxz * sxz);
+      vonmises[e] = sqrtf(fmaxf(0.0f, vm2));
+      // eigenpairs: cyclic Jacobi, at most 12 sweeps of the (1,2), (1,3), (2,3) rotations
+      float s11 = sxx, s22 = syy, s33 = szz, s12 = sxy, s23 = syz, s13 = sxz;
+      float v[3][3] = {{1.f, 0.f, 0.f}, {0.f, 1.f, 0.f}, {0.f, 0.f, 1.f}};
+      for (int it = 0; it < 12; ++it) {
+        if (fmaxf(fabsf(s12), fmaxf(fabsf(s23), fabsf(s13))) < 1.0e-9f) break;
+        jacobi_rotate(s11, s22, s12, s13, s23, v, 0, 1);
+        jacobi_rotate(s11, s33, s13, s12, s23, v, 0, 2);
+        jacobi_rotate(s22, s33, s23, s12, s13, v, 1, 2);
+      }
+      // descending order, columns of v swapped with their eigenvalues
+      auto swapcol = [&](int p, int q) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          const float t = v[r][p];
+          v[r][p] = v[r][q];
+          v[r][q] = t;
+        }
+      };
+      if (s11 < s22) { const float t = s11; s11 = s22; s22 = t; swapcol(0, 1); }
+      if (s22 < s33) { const float t = s22; s22 = s33; s33 = t; swapcol(1, 2); }
+      if (s11 < s22) { const float t = s11; s11 = s22; s22 = t; swapcol(0, 1); }
+      principal[3 * e] = s11, principal[3 * e + 1] = s22, principal[3 * e + 2] = s33;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) dmax[3 * e + r] = v[r][0], dmin[3 * e + r] = v[r][2];
+      l1[e] = fabsf(s11) + fabsf(s22) + fabsf(s33);
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) un[a][c] = un[a + 4][c];
+    }
   }
 }
 
@@ -154,9 +185,9 @@ template <typename TU>
 void launch_stress(const Grid& g, const TU* u, const float* density, float E, float nu, float dx, float dy, float dz,
                    int save_voigt, float* principal, float* vonmises, float* voigt, float* l1, float* dmax,
                    float* dmin, cudaStream_t st) {
-  const long long ne = g.nelem();
-  const int blocks = (int)std::max<long long>(1, std::min<long long>((ne + 255) / 256, 152LL * 16));
-  stress_kernel<TU><<<blocks, 256, 0, st>>>(g, u, density, E, nu, dx, dy, dz, save_voigt, principal, vonmises, voigt,
+  const long long items = (long long)((g.nx + 31) / 32) * ((g.ny + 3) / 4) * ((g.nz + kStressZ - 1) / kStressZ);
+  const int blocks = (int)std::min<long long>(items, 152LL * 64);
+  stress_kernel<TU><<<blocks, dim3(32, 4), 0, st>>>(g, u, density, E, nu, dx, dy, dz, save_voigt, principal, vonmises, voigt,
                                             l1, dmax, dmin);
 }
 
