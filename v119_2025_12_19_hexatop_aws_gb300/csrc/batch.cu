@@ -73,6 +73,7 @@ struct BLevel {
   std::vector<long long> off, eoff;
   long long ndof = 0, nelem = 0;
   T *fac = nullptr, *xa = nullptr, *xb = nullptr, *b = nullptr, *r = nullptr;
+  T* dn = nullptr;  // inverse diagonal per node of the smoothing instances
   T *dinv = nullptr, *p = nullptr, *q = nullptr, *z = nullptr, *w = nullptr;  // coarse scratch
   DevTable smooth;   // instances that smooth here
   DevTable coarse;   // instances whose coarsest level this is
@@ -141,8 +142,12 @@ void bvcycle(BatchCtx& B, BatchMG<T>& mg, int l, const T* b, T* xout) {
     prev = cur;
     cur = nx;
   };
-  launch_batch_jacobi0<T>(V.smooth.d, V.smooth.n(), V.smooth.vblocks, V.fac, mg.K, mg.quirk,
-                          mg.cheb ? mg.inv_theta : mg.omega, b, cur, B.s, c.st);
+  if (V.dn)
+    launch_batch_scale_nodes<T>(V.smooth.d, V.smooth.n(), V.smooth.vblocks, V.dn, mg.cheb ? mg.inv_theta : mg.omega, b,
+                                cur, B.s, c.st);
+  else
+    launch_batch_jacobi0<T>(V.smooth.d, V.smooth.n(), V.smooth.vblocks, V.fac, mg.K, mg.quirk,
+                            mg.cheb ? mg.inv_theta : mg.omega, b, cur, B.s, c.st);
   c.launches++;
   for (int s = 1; s < mg.nu1; ++s) {
     if (mg.cheb) {
@@ -304,6 +309,15 @@ bool build_batch_mg(Ctx& c, BatchMG<T>& mg, const std::vector<Grid>& g0, const s
     if (!upload(c, V.smooth, s + "s") || !upload(c, V.coarse, s + "c") || !upload(c, V.restr, s + "r") ||
         !upload(c, V.prolong, s + "p"))
       return false;
+    if (V.smooth.n() && node_dinv_ok(mg.K, mg.quirk)) {
+      V.dn = c.vec<T>(tag + std::to_string(l) + "dn", V.ndof / 3);
+      if (!V.dn) c.err.clear();  // formed from the factors instead
+      for (const BatchInst& b : V.smooth.h) {
+        if (!V.dn) break;
+        launch_node_dinv<T>(b.g, b.m, V.fac + b.eoff, mg.K, (T)b.sigma, V.dn + b.noff, c.st);
+        c.launches++;
+      }
+    }
     for (const BatchInst& b : V.coarse.h) {
       launch_diag<T>(b.g, b.m, V.fac + b.eoff, mg.K, mg.quirk, (T)b.sigma, nullptr, V.dinv + b.off, c.st);
       c.launches++;

@@ -76,6 +76,18 @@ void launch_node_bits(const uint8_t* fixed_dof, uint8_t* bits, long long nnode, 
 template <typename T>
 void launch_diag(const Grid& g, const Mask& m, const T* fac, const ModalK<T>& K, int quirk, T sigma,
                  T* diag, T* dinv, cudaStream_t st);
+// dn = 1/(dd[0]*fsum + sigma) per node, 0 at wholly fixed nodes: the inverse
+// diagonal where the three components share one entry (node_dinv_ok)
+template <typename T>
+void launch_node_dinv(const Grid& g, const Mask& m, const T* fac, const ModalK<T>& K, T sigma, T* dn, cudaStream_t st);
+template <typename T>
+inline bool node_dinv_ok(const ModalK<T>& K, int quirk) {
+  return quirk || (K.dd[0] == K.dd[1] && K.dd[1] == K.dd[2]);
+}
+// x = omega * dn * b on ncol columns (the first smoothing sweep from zero)
+template <typename T>
+void launch_scale_nodes(const T* dn, T omega, const T* b, T* x, long long nnode, const int* halt, cudaStream_t st,
+                        int ncol = 1);
 // max over the vector (non-negative entries), result into *dst (device)
 void launch_max(const double* v, long long n, const RedArgs& red, int nblocks, cudaStream_t st);
 // sums: dst = [a.b]  or [a.b, c.d]
@@ -327,6 +339,10 @@ void launch_batch_p_update(const BatchInst* in, int ninst, int nblocks, int node
 template <typename T>
 void launch_batch_dot(const BatchInst* in, int ninst, int nblocks, int node_sized, const T* a, const T* b,
                       const T* c, const T* d, const RedArgs& red, const PcgScalars* s, cudaStream_t st);
+// x = omega * dn * b per instance
+template <typename T>
+void launch_batch_scale_nodes(const BatchInst* in, int ninst, int nblocks, const T* dn, T omega, const T* b, T* x,
+                              const PcgScalars* s, cudaStream_t st);
 // dst = (T)(src * scale[id]) ; u += d / scale[id] (scale 0: left alone)
 template <typename T>
 void launch_batch_from64(const BatchInst* in, int ninst, int nblocks, T* dst, const double* src,

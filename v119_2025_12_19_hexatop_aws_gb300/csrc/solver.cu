@@ -126,6 +126,7 @@ struct Lev {
   T* b = nullptr;   // level right-hand side (coarse levels)
   T* r = nullptr;   // level residual
   T* dinv = nullptr, *p = nullptr, *q = nullptr, *z = nullptr;  // coarsest-level PCG
+  T* dn = nullptr;  // inverse diagonal per node (first sweep), null where the components differ
   T* w = nullptr;  // element-product scratch of the single-CTA coarse solve
   T* ainv = nullptr;  // dense inverse of the coarsest operator (small coarse grids)
   T* xw = nullptr, *bw = nullptr;  // W-cycle: second correction and its right-hand side
@@ -184,6 +185,15 @@ OpArgs<T> opargs(const Lev<T>& L, const ModalK<T>& K, int quirk, const T* x, con
   a.c1 = T(0);
   a.c2 = T(0);
   return a;
+}
+
+// First smoothing sweep from zero: x = omega D^-1 b on ncol columns.
+template <typename T>
+int first_sweep(Ctx& c, const Lev<T>& V, const ModalK<T>& K, int quirk, T omega, const T* b, T* x, const int* halt,
+                int ncol = 1) {
+  if (!V.dn) return launch_jacobi0<T>(V.g, V.m, V.fac, K, quirk, V.sigma, omega, b, x, halt, c.st, ncol);
+  launch_scale_nodes<T>(V.dn, omega, b, x, V.g.nnode(), halt, c.st, ncol);
+  return 1;
 }
 
 template <typename T>
@@ -311,6 +321,16 @@ void mg_set_shift(Ctx& c, MG<T>& mg, double sigma) {
   for (size_t l = 0; l < mg.L.size(); ++l) {
     mg.L[l].sigma = (T)s;
     s *= 8.0;  // row sums of P^T P
+    Lev<T>& V = mg.L[l];
+    if (l + 1 < mg.L.size() && node_dinv_ok(mg.K, mg.quirk)) {
+      V.dn = c.vec<T>((Is64<T>::v ? "mgdn64_" : "mgdn32_") + std::to_string(l), V.g.nnode());
+      if (V.dn) {
+        launch_node_dinv<T>(V.g, V.m, V.fac, mg.K, V.sigma, V.dn, c.st);
+        c.launches++;
+      } else {
+        c.err.clear();  // formed from the factors instead
+      }
+    }
   }
   Lev<T>& Lc = mg.L.back();
   launch_diag<T>(Lc.g, Lc.m, Lc.fac, mg.K, mg.quirk, Lc.sigma, nullptr, Lc.dinv, c.st);
@@ -381,8 +401,7 @@ bool vcycle(Ctx& c, MG<T>& mg, int l, const T* b, T* xout, const int* halt, cons
     cur = nx;
   };
   // the first sweep from zero is D^-1 b scaled by omega (damped Jacobi) or 1/theta (Chebyshev)
-  launch_jacobi0<T>(V.g, V.m, V.fac, mg.K, mg.quirk, V.sigma, cheb ? mg.inv_theta : mg.omega, b, cur, halt, c.st);
-  c.launches++;
+  c.launches += first_sweep<T>(c, V, mg.K, mg.quirk, cheb ? mg.inv_theta : mg.omega, b, cur, halt);
   for (int s = 1; s < mg.nu1; ++s) {
     if (cheb) {
       cheb_step(s);
@@ -489,8 +508,7 @@ void vcycle_cols(Ctx& c, MG<T>& mg, ColBufs<T>& cb, int l, const T* b, T* xout, 
     a.ncol = k;
     op<T>(c, mode, a);
   };
-  c.launches +=
-      launch_jacobi0<T>(V.g, V.m, V.fac, mg.K, mg.quirk, V.sigma, cheb ? mg.inv_theta : mg.omega, b, cur, halt, c.st, k);
+  c.launches += first_sweep<T>(c, V, mg.K, mg.quirk, cheb ? mg.inv_theta : mg.omega, b, cur, halt, k);
   for (int s = 1; s < mg.nu1; ++s) {
     T* nx = bufw(w++);
     if (cheb) {

@@ -163,6 +163,48 @@ void launch_diag(const Grid& g, const Mask& m, const T* fac, const ModalK<T>& K,
   diag_kernel<T><<<vec_blocks(g.nnode()), 256, 0, st>>>(g, m, fac, K, quirk, sigma, diag, dinv);
 }
 
+template <typename T>
+__global__ void node_dinv_kernel(Grid g, Mask m, const T* __restrict__ fac, T dd, T sigma, T* __restrict__ dn) {
+  const long long nn = g.nnode();
+  for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nn;
+       n += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(n % g.NX);
+    const long long t = n / g.NX;
+    const int j = (int)(t % g.NY), k = (int)(t / g.NY);
+    dn[n] = fixed_bits(g, m, i, j, k, n) == 7u ? T(0) : T(1) / fma(dd, node_factor_sum<T>(g, fac, i, j, k), sigma);
+  }
+}
+template <typename T>
+void launch_node_dinv(const Grid& g, const Mask& m, const T* fac, const ModalK<T>& K, T sigma, T* dn,
+                      cudaStream_t st) {
+  node_dinv_kernel<T><<<vec_blocks(g.nnode()), 256, 0, st>>>(g, m, fac, K.dd[0], sigma, dn);
+}
+
+// The first smoothing sweep with the inverse diagonal kept per node: 28/3 B a
+// DOF and no factor gather.  blockIdx.y: column.
+template <typename T>
+__global__ void __launch_bounds__(256) scale_nodes_kernel(const T* __restrict__ dn, T omega, const T* __restrict__ b,
+                                                          T* __restrict__ x, long long nn, const int* halt) {
+  if (halt && *((volatile const int*)halt)) return;
+  b += 3 * nn * blockIdx.y;
+  x += 3 * nn * blockIdx.y;
+  // three entries a thread, a block stride apart: 768 entries of 256 nodes per block step
+  for (long long n0 = (long long)blockIdx.x * 256; n0 < nn; n0 += (long long)gridDim.x * 256) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const long long q = 3 * n0 + c * 256 + threadIdx.x;
+      const long long n = n0 + (c * 256 + (int)threadIdx.x) / 3;
+      if (n < nn) x[q] = omega * dn[n] * b[q];
+    }
+  }
+}
+template <typename T>
+void launch_scale_nodes(const T* dn, T omega, const T* b, T* x, long long nnode, const int* halt, cudaStream_t st,
+                        int ncol) {
+  scale_nodes_kernel<T><<<dim3((unsigned)vec_blocks(nnode, 256, 152 * 16), (unsigned)ncol), 256, 0, st>>>(
+      dn, omega, b, x, nnode, halt);
+}
+
 __global__ void max_kernel(const double* __restrict__ v, long long n, RedArgs red) {
   double mx = -INFINITY;
   bool bad = false;
@@ -643,6 +685,26 @@ void launch_batch_dot(const BatchInst* in, int ninst, int nblocks, int node_size
 }
 
 template <typename T>
+__global__ void batch_scale_nodes_kernel(const BatchInst* in, int ninst, const T* __restrict__ dn, T omega,
+                                         const T* __restrict__ b, T* __restrict__ x, const PcgScalars* s) {
+  const BatchInst& I = in[batch_find_vec(in, ninst, blockIdx.x)];
+  if (inst_halted(s, I.id)) return;
+  const long long nn = I.g.nnode();
+  for (long long n0 = (long long)(blockIdx.x - I.vblk0) * 256; n0 < nn; n0 += (long long)I.vnblk * 256) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const long long q = 3 * n0 + c * 256 + threadIdx.x, n = n0 + (c * 256 + (int)threadIdx.x) / 3;
+      if (n < nn) x[I.off + q] = omega * dn[I.noff + n] * b[I.off + q];
+    }
+  }
+}
+template <typename T>
+void launch_batch_scale_nodes(const BatchInst* in, int ninst, int nblocks, const T* dn, T omega, const T* b, T* x,
+                              const PcgScalars* s, cudaStream_t st) {
+  batch_scale_nodes_kernel<T><<<nblocks, 256, 0, st>>>(in, ninst, dn, omega, b, x, s);
+}
+
+template <typename T>
 __global__ void batch_from64_kernel(const BatchInst* in, int ninst, T* __restrict__ dst,
                                     const double* __restrict__ src, const double* scale) {
   const BatchSeg sg = batch_seg(in, ninst, 0);
@@ -704,6 +766,10 @@ int vec_batch_plan(BatchInst* in, int n, int unit, int max_blocks) {
 #define INST(T)                                                                                 \
   template void launch_fill<T>(T*, T, long long, cudaStream_t);                                 \
   template void launch_copy<T>(T*, const T*, long long, cudaStream_t);                          \
+  template void launch_node_dinv<T>(const Grid&, const Mask&, const T*, const ModalK<T>&, T, T*, cudaStream_t);  \
+  template void launch_scale_nodes<T>(const T*, T, const T*, T*, long long, const int*, cudaStream_t, int);      \
+  template void launch_batch_scale_nodes<T>(const BatchInst*, int, int, const T*, T, const T*, T*,               \
+                                            const PcgScalars*, cudaStream_t);                                    \
   template void launch_diag<T>(const Grid&, const Mask&, const T*, const ModalK<T>&, int, T, T*, \
                                T*, cudaStream_t);                                               \
   template void launch_dot<T>(const T*, const T*, const T*, const T*, long long, const RedArgs&, \
