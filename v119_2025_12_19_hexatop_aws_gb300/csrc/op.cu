@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 #include "hexa_common.cuh"
@@ -288,6 +289,189 @@ __device__ __forceinline__ void element_modal<float>(const ModalK<float>& K, con
 }
 #endif
 
+// ------------------------------------------ FP64 element product in integers
+// The FP64 operator is bound by FP64 issue: 2 instructions per clock and SM,
+// against 64 or more integer ones.  An element's product is therefore formed in
+// 64-bit fixed point, scaled per element, and only the sums over elements (with
+// the factors) stay FP64: 36 FP64 instructions an element layer instead of 190.
+//   * a node layer's corner values become integers at the layer's largest
+//     exponent (58 bits; FP64's 53 are exact down to 2^-5 of the largest), and
+//     the butterflies on them are exact;
+//   * the strain modes are normalised by a common shift (61 bits), so the
+//     precision follows the strains, not the rigid motion they were taken from;
+//   * the modal blocks multiply as two 32-bit halves (vh ch, vh cl, vl ch
+//     accumulated in 64 bits; the dropped vl cl is below 2^-60 of the largest
+//     mode times the largest coefficient), the inverse butterflies are exact.
+// Each rounding is relative to the element's largest mode and below 2^-58 of
+// it, where FP64 rounds at 2^-53 of every intermediate sum.  Chosen when the
+// smallest non-zero modal coefficient is within 2^-6 of the largest (every brick
+// and nu in ordinary use; not nu near 0.5 or needle elements), else the FP64
+// form.  The norm of the true residual (OP_RESID_NORM), which a solve reports,
+// stays in the FP64 form: a caller who recomputes it in FP64 at the rounding
+// limit finds that arithmetic's rounding in it (single solves, batches).  A
+// non-finite corner makes the element's product NaN.
+// 256x128x128 product: 0.60 ms, 1.90 in FP64 (8 warps and 0.82 ms with the
+// layers prefetched into registers; 14 and 16 warps 0.63 and 0.64); against
+// quad precision its error is 0.90 to 1.00 of the FP64 form's on random
+// displacements and 0.04 to 0.4 on smooth ones, where FP64 loses the strains to
+// the rigid motion.
+constexpr int kFixedWarps = 12;  // one CTA per SM at 168 registers
+struct FixedK {
+  int h[8][3][3], l[8][3][3];  // B = (h 2^32 + l) 2^-exp, l signed
+  int exp;
+  bool ok;
+};
+static FixedK fixed_blocks(const ModalK<double>& K) {
+  FixedK F;
+  double mx = 0.0, mn = 1e300;
+  for (int q = 0; q < 8; ++q)
+    for (int c = 0; c < 3; ++c)
+      for (int d = 0; d < 3; ++d)
+        if (modal_nz(q, c, d)) {
+          const double v = std::fabs(K.B[q][c][d]);
+          mx = std::max(mx, v);
+        }
+  for (int q = 0; q < 8; ++q)
+    for (int c = 0; c < 3; ++c)
+      for (int d = 0; d < 3; ++d) {
+        const double v = std::fabs(K.B[q][c][d]);
+        if (v > 1e-12 * mx) mn = std::min(mn, v);  // below: zero but for the quadrature's rounding
+      }
+  F.ok = std::isfinite(mx) && mx > 0.0 && mn >= mx / 64.0;
+  int e = 0;
+  std::frexp(mx, &e);  // mx < 2^e
+  F.exp = 61 - e;
+  for (int q = 0; q < 8; ++q)
+    for (int c = 0; c < 3; ++c)
+      for (int d = 0; d < 3; ++d) {
+        const long long v = F.ok ? std::llrint(std::ldexp(K.B[q][c][d], F.exp)) : 0;
+        F.l[q][c][d] = (int)(v & 0xffffffffLL);
+        F.h[q][c][d] = (int)((v - F.l[q][c][d]) >> 32);
+      }
+  return F;
+}
+
+// Corner values -> xy-modal integers; returns the layer's exponent field (the
+// integers are in units of 2^(E - 1080)), 0x7ff when a value is not finite.
+__device__ __forceinline__ int fixed_layer(const double (&v)[4][3], long long (&m)[4][3]) {
+  unsigned mx = 0;
+#pragma unroll
+  for (int cc = 0; cc < 4; ++cc)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) mx = max(mx, (unsigned)__double2hiint(v[cc][c]) & 0x7fffffffu);
+  const int E = (int)(mx >> 20);
+  long long q[4][3];
+#pragma unroll
+  for (int cc = 0; cc < 4; ++cc)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int hi = __double2hiint(v[cc][c]);
+      const int e = (hi >> 20) & 0x7ff;
+      const unsigned long long mant =
+          ((unsigned long long)(unsigned)((hi & 0xfffff) | 0x100000) << 32 | (unsigned)__double2loint(v[cc][c])) << 5;
+      const int d = e == 0 ? 63 : min(E - e, 63);  // zero and subnormal values: 0
+      q[cc][c] = (long long)(mant >> d) ^ (long long)(hi >> 31);  // negative: one's complement, one unit below
+    }
+  xy_forward<long long>(q, m);
+  return E;
+}
+
+// q rounded to a double, by integer operations: the conversion instruction runs
+// on the FP64 pipe (0.80 ms against 0.60 for the 256x128x128 product).  The
+// leading bit is looked for in the high word; values below 2^32 units shift
+// their low word up.  A carry out of the mantissa runs into the exponent.
+__device__ __forceinline__ double fixed_to_double(long long q) {
+  const unsigned s = (unsigned)((int)(q >> 32) >> 31);
+  unsigned uh = (unsigned)(q >> 32) ^ s, ul = (unsigned)q ^ s;
+  int ex = 1085;
+  if (uh == 0) {
+    uh = ul, ul = 0, ex = 1053;
+    if (uh == 0) return 0.0;
+  }
+  const int z = __clz((int)uh);
+  const unsigned th = __funnelshift_l(ul, uh, z), tl = ul << z;
+  const unsigned long long b =
+      (((unsigned long long)(th >> 11) << 32) | __funnelshift_r(tl, th, 11)) + ((tl >> 10) & 1u);
+  return __hiloint2double((int)((unsigned)(b >> 32) + ((unsigned)(ex - z) << 20)) | (int)(s & 0x80000000u),
+                          (int)(unsigned)b);
+}
+
+// f * 2^x
+__device__ __forceinline__ double scale_exp(double f, int x) {
+  const int hi = __double2hiint(f), e = (hi >> 20) & 0x7ff;
+  if (e != 0 && e != 0x7ff && e + x > 0 && e + x < 0x7ff)
+    return __hiloint2double(hi + x * (1 << 20), __double2loint(f));
+  return scalbn(f, x);  // zero, subnormal, non-finite or out of range
+}
+
+// One element: lower and upper xy-modal layers -> the corner values of K0 u_e in
+// integers (lo: lower layer, hi: upper) and the factor that scales them.
+template <bool LOWER>
+__device__ __forceinline__ double element_fixed(const FixedK& K, const long long (&L)[4][3], int eL,
+                                                const long long (&U)[4][3], int eU, double f, long long (&lo)[4][3],
+                                                long long (&hi)[4][3]) {
+  const int E = max(eL, eU), dl = min(E - eL, 63), du = min(E - eU, 63);
+  long long h[8][3];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const long long a = L[m][c] >> dl, b = U[m][c] >> du;
+      h[m][c] = a + b;
+      h[m + 4][c] = b - a;
+    }
+  unsigned acc = 0;
+#pragma unroll
+  for (int m = 1; m < 8; ++m)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int t = (int)(h[m][c] >> 32);
+      acc |= (unsigned)(t ^ (t >> 31));
+    }
+  const int n = min(__clz((int)acc), 31) - 3;  // |h| < 2^61 before and after: mode sums of 8 values below 2^58
+  int vh[8][3], vl[8][3];
+#pragma unroll
+  for (int m = 1; m < 8; ++m)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const long long t = h[m][c] << n;
+      vl[m][c] = (int)t;
+      vh[m][c] = (int)(t >> 32) - (vl[m][c] >> 31);
+    }
+  long long w[8][3];
+#pragma unroll
+  for (int m = 0; m < 8; ++m)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int q = m ^ (1 << c);
+      long long A = 0, M = 0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (modal_nz(q, c, d)) {
+          const int m2 = q ^ (1 << d);
+          A += (long long)vh[m2][d] * K.h[q][c][d];
+          M += (long long)vh[m2][d] * K.l[q][c][d];
+          M += (long long)vl[m2][d] * K.h[q][c][d];
+        }
+      w[m][c] = A + (M >> 32);
+    }
+  long long a[4][3];
+  if (LOWER) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) a[m][c] = w[m][c] - w[m + 4][c];
+    xy_inverse<long long>(a, lo);
+  }
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) a[m][c] = w[m][c] + w[m + 4][c];
+  xy_inverse<long long>(a, hi);
+  const double fs = scale_exp(f, E - 1016 - n - K.exp);  // units 2^(E - 1080), 2^-n, coefficients 2^-exp, >> 64
+  return E == 0x7ff ? __hiloint2double(0x7ff80000, 0) : fs;
+}
+
 // CTA height in warps.  FP32: 16 warps, one CTA per SM (127 registers); 8-warp
 // CTAs two per SM measured 5 % slower on the 384x192x192 Chebyshev step
 // (359 us against 340 us), the larger halo outweighing the shorter barriers.
@@ -340,8 +524,8 @@ __device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
 #endif
 __device__ __forceinline__ void pair_barrier(int b) { asm volatile("bar.sync %0, 64;" ::"r"(b) : "memory"); }
 
-template <typename T, int MODE, int TYW, typename IX, typename A, bool INTERIOR = false>
-__device__ __forceinline__ void op_item(const A& a, int tx, int ty, int chunk,
+template <typename T, int MODE, int TYW, typename IX, bool FX, typename A, bool INTERIOR = false>
+__device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, int ty, int chunk,
                                         T (&xch)[2][TYW][32][4],
                                         double& acc0, long long co) {
   // the _DOT forms of the smoothing steps also sum b.y
@@ -418,22 +602,38 @@ __device__ __forceinline__ void op_item(const A& a, int tx, int ty, int chunk,
         for (int c = 0; c < 3; ++c) v[cc][c] = ((m >> (3 * cc + c)) & 1u) ? T(0) : v[cc][c];
     }
   };
-  T Lm[4][3], carry[4][3], xown[3];
+  // FX: integer layers and their exponent, and a carry in corner values
+  using M = typename std::conditional<FX, long long, T>::type;
+  M Lm[4][3];
+  int eL = 0;
+  T carry[4][3], xown[3];
   T fprev;
   {
     T raw[4][3];
     load_corners<T, IX, INTERIOR>(g, ca, x, k0 - 1, raw);
     drop_fixed(raw, load_bits(k0 - 1));
-    T Lprev[4][3];
-    xy_forward<T>(raw, Lprev);
+    M Lprev[4][3];
+    int ep = 0;
+    if constexpr (FX) ep = fixed_layer(raw, Lprev);
+    else xy_forward<T>(raw, Lprev);
     load_corners<T, IX, INTERIOR>(g, ca, x, k0, raw);
     drop_fixed(raw, load_bits(k0));
 #pragma unroll
     for (int c = 0; c < 3; ++c) xown[c] = raw[3][c];
-    xy_forward<T>(raw, Lm);
     fprev = facload(k0 - 1);
-    T lo[4][3];
-    element_modal<T>(a.K, Lprev, Lm, fprev, lo, carry);
+    if constexpr (FX) {
+      eL = fixed_layer(raw, Lm);
+      M none[4][3], up[4][3];
+      const T fs = element_fixed<false>(*fk, Lprev, ep, Lm, eL, fprev, none, up);
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) carry[cc][c] = fs * fixed_to_double(up[cc][c]);
+    } else {
+      xy_forward<T>(raw, Lm);
+      T lo[4][3];
+      element_modal<T>(a.K, Lprev, Lm, fprev, lo, carry);
+    }
   }
   // b and the previous iterate at the own node are loaded one layer ahead, so
   // their DRAM latency hides behind the next layer's element work
@@ -467,55 +667,81 @@ __device__ __forceinline__ void op_item(const A& a, int tx, int ty, int chunk,
   // 384x192x192); the apply forms are faster with the loads first (0.1977
   // against 0.2011).
   constexpr bool EARLY = NEED_B;
+  constexpr bool PRE = !FX;  // the integer form is far from load-bound, and its registers are
 
   // sums of this item in the kernel's own precision (one item is at most a
   // few dozen layers per thread), folded into the FP64 accumulator at the end:
   // FP64 arithmetic in the FP32 kernels would run at GB300's FP64 rate
   T accT = T(0);
   T nraw[4][3];
-  load_corners<T, IX, INTERIOR>(g, ca, x, k0 + 1, nraw);
-  unsigned nbits = load_bits(k0 + 1);
+  unsigned nbits = 0;
+  if (PRE) {
+    load_corners<T, IX, INTERIOR>(g, ca, x, k0 + 1, nraw);
+    nbits = load_bits(k0 + 1);
+  }
   T fnext = facload(k0);
 
   // three layers per unrolled step for the Chebyshev forms, two for the rest
   // (on the 384x192x192 grid: Chebyshev step 0.2191 ms at 3 against 0.2248
   // at 2 and 0.2475 at 1; Jacobi step 0.2006 at 3, 0.1983 at 2)
-#pragma unroll(BM == OP_CHEB2 ? 3 : 2)
+#pragma unroll(FX ? 1 : (BM == OP_CHEB2 ? 3 : 2))
   for (int k = k0; k < k1; ++k) {
+    if (!PRE) {
+      load_corners<T, IX, INTERIOR>(g, ca, x, k + 1, nraw);
+      nbits = load_bits(k + 1);
+    }
     drop_fixed(nraw, nbits);
     const T f = fnext;
     T bk[3], pk3[3], xup[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) bk[c] = bnext[c], pk3[c] = pnext[c], xup[c] = nraw[3][c];
-    T Um[4][3];
-    if (EARLY) xy_forward<T>(nraw, Um);
+    M Um[4][3];
+    int eU = 0;
+    if constexpr (FX) eU = fixed_layer(nraw, Um);
+    else if (EARLY) xy_forward<T>(nraw, Um);
     T raw[4][3];
-    if (!EARLY) {
+    if (!EARLY && !FX) {
 #pragma unroll
       for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
         for (int c = 0; c < 3; ++c) raw[cc][c] = nraw[cc][c];
     }
     if (k + 1 < k1) {  // prefetch the next layer
-      load_corners<T, IX, INTERIOR>(g, ca, x, k + 2, nraw);
-      nbits = load_bits(k + 2);
+      if (PRE) {
+        load_corners<T, IX, INTERIOR>(g, ca, x, k + 2, nraw);
+        nbits = load_bits(k + 2);
+      }
       fnext = facload(k + 1);
       if (NEED_B || NEED_P) load_bp(k + 1);
     }
     touch_l2(k);
-    if (!EARLY) xy_forward<T>(raw, Um);
-    T lo[4][3], hi[4][3];
-    element_modal<T>(a.K, Lm, Um, f, lo, hi);
-    add_carry<T>(lo, carry);
+    T cv[4][3];
+    if constexpr (FX) {
+      M lo[4][3], hi[4][3];
+      const T fs = element_fixed<true>(*fk, Lm, eL, Um, eU, f, lo, hi);
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          cv[cc][c] = fma(fs, fixed_to_double(lo[cc][c]), carry[cc][c]);
+          carry[cc][c] = fs * fixed_to_double(hi[cc][c]);
+        }
+      eL = eU;
+    } else {
+      if (!EARLY) xy_forward<T>(raw, Um);
+      T lo[4][3], hi[4][3];
+      element_modal<T>(a.K, Lm, Um, f, lo, hi);
+      add_carry<T>(lo, carry);
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) carry[m][c] = hi[m][c];
+      xy_inverse<T>(lo, cv);
+    }
 #pragma unroll
     for (int m = 0; m < 4; ++m)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        carry[m][c] = hi[m][c];
-        Lm[m][c] = Um[m][c];
-      }
-    T cv[4][3];
-    xy_inverse<T>(lo, cv);
+      for (int c = 0; c < 3; ++c) Lm[m][c] = Um[m][c];
     // node (i0+p, j0+q) = c11(p,q) + c01(p+1,q) + c10(p,q+1) + c00(p+1,q+1)
     T T1[3], T0[3];
 #pragma unroll
@@ -617,14 +843,39 @@ __global__ void __launch_bounds__(32 * TYW, op_min_ctas<T>()) op_kernel(const Op
     const int chunk = item / nxy, t = item - chunk * nxy;
     const int ty = t / a.tiles_x, tx = t - ty * a.tiles_x;
     if (MULTI) {  // every column of a multi-column apply reuses the item's factors from L1
-      for (int col = 0; col < a.ncol; ++col) op_item<T, MODE, TYW, IX>(a, tx, ty, chunk, xch, acc0, col * a.g.ndof());
+      for (int col = 0; col < a.ncol; ++col) op_item<T, MODE, TYW, IX, false>(a, nullptr, tx, ty, chunk, xch, acc0, col * a.g.ndof());
     } else if (HEXA_OP_INTERIOR && tile_interior<TYW>(a.g, tx, ty)) {
-      op_item<T, MODE, TYW, IX, OpArgs<T>, true>(a, tx, ty, chunk, xch, acc0, 0);
+      op_item<T, MODE, TYW, IX, false, OpArgs<T>, true>(a, nullptr, tx, ty, chunk, xch, acc0, 0);
     } else {
-      op_item<T, MODE, TYW, IX>(a, tx, ty, chunk, xch, acc0, 0);
+      op_item<T, MODE, TYW, IX, false>(a, nullptr, tx, ty, chunk, xch, acc0, 0);
     }
   }
   if (MODE == OP_APPLY_DOT || MODE == OP_RESID_NORM || MODE == OP_JACOBI_DOT || MODE == OP_CHEB2_DOT) {
+    double v[1] = {acc0};
+    block_reduce_finalize<1>(a.red, v);
+  }
+}
+
+// The same over the integer element product (FP64, 32-bit indices).
+template <int MODE, int TYW, bool MULTI>
+__global__ void __launch_bounds__(32 * TYW, 1) op_fixed_kernel(const __grid_constant__ OpArgs<double> a,
+                                                               const __grid_constant__ FixedK fk) {
+  if (a.halt && *((volatile const int*)a.halt)) return;
+  __shared__ __align__(16) double xch[2][TYW][32][4];
+  double acc0 = 0.0;
+  const int nxy = a.tiles_x * a.tiles_y;
+  const int items = nxy * a.nchunks;
+  for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    const int chunk = item / nxy, t = item - chunk * nxy;
+    const int ty = t / a.tiles_x, tx = t - ty * a.tiles_x;
+    if (MULTI) {
+      for (int col = 0; col < a.ncol; ++col)
+        op_item<double, MODE, TYW, int, true>(a, &fk, tx, ty, chunk, xch, acc0, col * a.g.ndof());
+    } else {
+      op_item<double, MODE, TYW, int, true>(a, &fk, tx, ty, chunk, xch, acc0, 0);
+    }
+  }
+  if (MODE == OP_APPLY_DOT || MODE == OP_JACOBI_DOT || MODE == OP_CHEB2_DOT) {
     double v[1] = {acc0};
     block_reduce_finalize<1>(a.red, v);
   }
@@ -1081,6 +1332,7 @@ template <typename T>
 int op_pick_kchunk(const Grid& g) {
   int tx, ty, nch;
   op_tiles<T>(g, 1, &tx, &ty, &nch);
+  if (sizeof(T) == 8) ty = (g.NY + kFixedWarps - 2) / (kFixedWarps - 1);
   const long long tiles = (long long)tx * ty, ctas = resident_ctas<T>(OP_CHEB2);
   if (sizeof(T) == 4 && op_form() == 1) {  // the staged form fills its ring over an item's layers: at least 16
     long long chunks = (8 * ctas + tiles - 1) / tiles;
@@ -1155,6 +1407,36 @@ static void launch_op_tma(int mode, OpArgs<float>& a, bool i32, cudaStream_t st)
 #undef HEXA_OPT_CASE
 }
 
+static bool launch_op_fixed(int mode, const OpArgs<double>& a0, const FixedK& fk, cudaStream_t st) {
+  constexpr int TYW = kFixedWarps;
+  OpArgs<double> a = a0;
+  a.tiles_y = (a.g.NY + TYW - 2) / (TYW - 1);
+  const long long items = (long long)a.tiles_x * a.tiles_y * a.nchunks;
+  const int grid = (int)std::min<long long>(items, 152);
+  const dim3 block(32, TYW);
+#define HEXA_FX_CASE(M, MULTI) \
+  case M: op_fixed_kernel<M, TYW, MULTI><<<grid, block, 0, st>>>(a, fk); return true;
+  if (a.ncol > 1) switch (mode) {
+      HEXA_FX_CASE(OP_APPLY, true)
+      HEXA_FX_CASE(OP_RESID, true)
+      HEXA_FX_CASE(OP_JACOBI, true)
+      HEXA_FX_CASE(OP_CHEB2, true)
+      default: return false;
+    }
+  switch (mode) {
+    HEXA_FX_CASE(OP_APPLY, false)
+    HEXA_FX_CASE(OP_APPLY_DOT, false)
+    HEXA_FX_CASE(OP_RESID, false)
+    HEXA_FX_CASE(OP_JACOBI, false)
+    HEXA_FX_CASE(OP_CHEB2, false)
+    HEXA_FX_CASE(OP_JACOBI_DOT, false)
+    HEXA_FX_CASE(OP_CHEB2_DOT, false)
+    HEXA_FX_CASE(OP_APPLY_MASK, false)
+    default: return false;
+  }
+#undef HEXA_FX_CASE
+}
+
 template <typename T>
 void launch_op(int mode, const OpArgs<T>& a0, cudaStream_t st) {
   constexpr int TYW = op_tyw<T>();
@@ -1168,6 +1450,12 @@ void launch_op(int mode, const OpArgs<T>& a0, cudaStream_t st) {
     if (a.ncol <= 1 && op_form() == 1) {
       launch_op_tma(mode, a, i32, st);
       return;
+    }
+  }
+  if constexpr (sizeof(T) == 8) {
+    if (i32) {
+      const FixedK fk = fixed_blocks(a.K);
+      if (fk.ok && launch_op_fixed(mode, a, fk, st)) return;
     }
   }
   if (a.ncol > 1) {  // multi-column forms (no reductions): apply, residual and the two smoothing steps
@@ -1253,7 +1541,7 @@ __global__ void __launch_bounds__(32 * TYW, op_min_ctas<T>()) op_batch_kernel(co
   for (int item = local; item < items; item += nb) {
     const int chunk = item / nxy, t = item - chunk * nxy;
     const int ty = t / txs, tx = t - ty * txs;
-    op_item<T, MODE, TYW, IX>(ia, tx, ty, chunk, xch, acc0, 0);
+    op_item<T, MODE, TYW, IX, false>(ia, nullptr, tx, ty, chunk, xch, acc0, 0);
   }
   if (MODE == OP_APPLY_DOT || MODE == OP_RESID_NORM) {
     double v[1] = {acc0};
