@@ -34,6 +34,7 @@ def test_cut_among_equal_densities(ctx, rng, ties, cut):
     assert st["culled"] == k and st["active_count"] == ne
     assert np.array_equal(d, ref)
     dev = torch.ones(ne, device="cuda")
+    torch.cuda.synchronize()  # the context works on a stream of its own
     update_density_gpu(_lib.make_grid(*dims), dev, torch.from_numpy(rho).cuda(), None, torch.from_numpy(orig).cuda(), p,
                        ctx=ctx)
     assert np.array_equal(dev.cpu().numpy(), ref)

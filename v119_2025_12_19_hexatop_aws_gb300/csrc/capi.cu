@@ -361,7 +361,7 @@ static int time_operator_t(hexa_ctx* h, const hexa_grid* g, const hexa_bc* bc, d
     a.c1 = T(0.5);
     a.c2 = T(0.3);
   }
-  a.kchunk = op_pick_kchunk<T>(G);
+  a.kchunk = op_pick_kchunk<T>(G, mode);
   a.diag_quirk = 1;
   const long long nb = op_num_blocks<T>(G, a.kchunk);
   if (!c.ensure_partials((size_t)nb * 2 + 64)) return HEXA_ERR_NOMEM;

@@ -52,9 +52,9 @@ bool op_staged_form();
 bool op_take_wait_error(cudaStream_t st);
 template <typename T>
 long long op_num_blocks(const Grid& g, int kchunk);
-// node layers per work item (see op.cu)
+// node layers per work item of a mode's launches (see op.cu)
 template <typename T>
-int op_pick_kchunk(const Grid& g);
+int op_pick_kchunk(const Grid& g, int mode = OP_APPLY);
 ModalK<float> modal_to_f32(const ModalK<double>& K);
 
 // ------------------------------------------------------------ vector passes

@@ -524,7 +524,7 @@ __device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
 #endif
 __device__ __forceinline__ void pair_barrier(int b) { asm volatile("bar.sync %0, 64;" ::"r"(b) : "memory"); }
 
-template <typename T, int MODE, int TYW, typename IX, bool FX, typename A, bool INTERIOR = false>
+template <typename T, int MODE, int TYW, typename IX, bool FX, bool TOUCH = false, typename A, bool INTERIOR = false>
 __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, int ty, int chunk,
                                         T (&xch)[2][TYW][32][4],
                                         double& acc0, long long co) {
@@ -654,9 +654,10 @@ __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, in
   // x, b and the previous iterate two layers past the register prefetch, into
   // L2: 384x192x192 Chebyshev step 0.2207 -> 0.2160 ms, residual 0.2086 ->
   // 0.2032, apply with p.Ap 0.2022 -> 0.1978; three to six layers gain less.
+  // Only in the kernels of grids whose vectors overflow L2 (launch_op).
   const IX touch0 = (IX)3 * ((IX)min(in, g.NX - 1) + (IX)g.NX * min(jn, g.NY - 1));
   auto touch_l2 = [&](int k) {
-    if (k + 3 >= k1) return;
+    if (!TOUCH || k + 3 >= k1) return;
     const IX at = touch0 + (IX)3 * nplane * (IX)(k + 2);
     asm volatile("prefetch.global.L2 [%0];" ::"l"(x + (at + (IX)3 * nplane)));
     if (NEED_B) asm volatile("prefetch.global.L2 [%0];" ::"l"(bv + at));
@@ -830,7 +831,7 @@ __device__ __forceinline__ bool tile_interior(const Grid& g, int tx, int ty) {
   return i0 >= 1 && i0 + 31 <= g.NX - 1 && j0 >= 1 && j0 + TYW - 1 <= g.NY - 1;
 }
 
-template <typename T, int MODE, int TYW, typename IX, bool MULTI>
+template <typename T, int MODE, int TYW, typename IX, bool MULTI, bool TOUCH = false>
 __global__ void __launch_bounds__(32 * TYW, op_min_ctas<T>()) op_kernel(const OpArgs<T> a) {
   if (a.halt && *((volatile const int*)a.halt)) return;
   __shared__ __align__(16) T xch[2][TYW][32][4];
@@ -845,9 +846,9 @@ __global__ void __launch_bounds__(32 * TYW, op_min_ctas<T>()) op_kernel(const Op
     if (MULTI) {  // every column of a multi-column apply reuses the item's factors from L1
       for (int col = 0; col < a.ncol; ++col) op_item<T, MODE, TYW, IX, false>(a, nullptr, tx, ty, chunk, xch, acc0, col * a.g.ndof());
     } else if (HEXA_OP_INTERIOR && tile_interior<TYW>(a.g, tx, ty)) {
-      op_item<T, MODE, TYW, IX, false, OpArgs<T>, true>(a, nullptr, tx, ty, chunk, xch, acc0, 0);
+      op_item<T, MODE, TYW, IX, false, TOUCH, OpArgs<T>, true>(a, nullptr, tx, ty, chunk, xch, acc0, 0);
     } else {
-      op_item<T, MODE, TYW, IX, false>(a, nullptr, tx, ty, chunk, xch, acc0, 0);
+      op_item<T, MODE, TYW, IX, false, TOUCH>(a, nullptr, tx, ty, chunk, xch, acc0, 0);
     }
   }
   if (MODE == OP_APPLY_DOT || MODE == OP_RESID_NORM || MODE == OP_JACOBI_DOT || MODE == OP_CHEB2_DOT) {
@@ -1329,10 +1330,10 @@ constexpr double op_item_start() { return sizeof(T) == 8 ? 0.6 : 2.0; }
 // layers took 13.6 us, 13 CTAs of one layer 5 us); large ones keep long
 // chunks that divide evenly over the CTAs.
 template <typename T>
-int op_pick_kchunk(const Grid& g) {
+int op_pick_kchunk(const Grid& g, int mode) {
   int tx, ty, nch;
   op_tiles<T>(g, 1, &tx, &ty, &nch);
-  if (sizeof(T) == 8) ty = (g.NY + kFixedWarps - 2) / (kFixedWarps - 1);
+  if (sizeof(T) == 8 && mode != OP_RESID_NORM) ty = (g.NY + kFixedWarps - 2) / (kFixedWarps - 1);
   const long long tiles = (long long)tx * ty, ctas = resident_ctas<T>(OP_CHEB2);
   if (sizeof(T) == 4 && op_form() == 1) {  // the staged form fills its ring over an item's layers: at least 16
     long long chunks = (8 * ctas + tiles - 1) / tiles;
@@ -1474,9 +1475,16 @@ void launch_op(int mode, const OpArgs<T>& a0, cudaStream_t st) {
     }
     return;
   }
+  // FP32 vectors of which one overflows L2 are prefetched into it ahead of the
+  // march: 2 to 3% of a launch at 384x192x192 (172 MB a vector); at 192^3 (86 MB)
+  // the same prefetch cost a multigrid solve 2% (91.3 -> 93.6 ms), its
+  // instructions alone, switched off at run time, 1.8%.
+  constexpr bool F32 = sizeof(T) == 4;
+  const bool touch = F32 && a.g.ndof() * (long long)sizeof(T) > (120LL << 20);
 #define HEXA_OP_CASE(M)                                                              \
   case M:                                                                           \
-    if (i32) op_kernel<T, M, TYW, int, false><<<grid, block, 0, st>>>(a);           \
+    if (i32 && touch) op_kernel<T, M, TYW, int, false, F32><<<grid, block, 0, st>>>(a);  \
+    else if (i32) op_kernel<T, M, TYW, int, false><<<grid, block, 0, st>>>(a);      \
     else op_kernel<T, M, TYW, long long, false><<<grid, block, 0, st>>>(a);         \
     break;
   switch (mode) {
@@ -1632,8 +1640,8 @@ template void launch_op<double>(int, const OpArgs<double>&, cudaStream_t);
 template void launch_op<float>(int, const OpArgs<float>&, cudaStream_t);
 template long long op_num_blocks<double>(const Grid&, int);
 template long long op_num_blocks<float>(const Grid&, int);
-template int op_pick_kchunk<double>(const Grid&);
-template int op_pick_kchunk<float>(const Grid&);
+template int op_pick_kchunk<double>(const Grid&, int);
+template int op_pick_kchunk<float>(const Grid&, int);
 template ModalK<float> cast_modal<float>(const ModalK<double>&);
 template ModalK<double> cast_modal<double>(const ModalK<double>&);
 

@@ -101,8 +101,8 @@ template <typename T>
 struct Is64 { static constexpr bool v = sizeof(T) == 8; };
 
 template <typename T>
-int pick_kchunk(const Grid& g) {
-  return op_pick_kchunk<T>(g);
+int pick_kchunk(const Grid& g, int mode = OP_APPLY) {
+  return op_pick_kchunk<T>(g, mode);
 }
 
 RedArgs red(Ctx& c, int op, int nsum, PcgScalars* s, double* dst = nullptr) {
@@ -748,7 +748,7 @@ double true_residual_norm(Ctx& c, const Problem& P, const ModalK<double>& K64, i
   L.m = P.m;
   L.fac = const_cast<double*>(P.fac64);
   L.sigma = sigma;
-  L.kchunk = pick_kchunk<double>(P.g);
+  L.kchunk = pick_kchunk<double>(P.g, OP_RESID_NORM);
   op<double>(c, OP_RESID_NORM, opargs<double>(L, K64, quirk, u, P.f64, r64, 0.0, nullptr, red(c, FIN_STORE, 1, nullptr, c.dscal + 8)));
   cudaMemcpyAsync(c.hscal + 8, c.dscal + 8, sizeof(double), cudaMemcpyDeviceToHost, c.st);
   cudaStreamSynchronize(c.st);
@@ -793,7 +793,8 @@ bool setup_common(Ctx& c, const Problem& P, const hexa_solve_params& prm, ModalK
   const long long n = P.g.ndof();
   double* diag = c.vec<double>("diag64", n);
   if (!diag) return false;
-  const long long maxblocks = op_num_blocks<double>(P.g, pick_kchunk<double>(P.g)) + 8;
+  const int kc = std::min(pick_kchunk<double>(P.g), pick_kchunk<double>(P.g, OP_RESID_NORM));
+  const long long maxblocks = op_num_blocks<double>(P.g, kc) + 8;
   if (!c.ensure_partials((size_t)std::max<long long>(maxblocks * 2, kRedBlocks * 2 + 16) + 4096)) return false;
   launch_diag<double>(P.g, P.m, P.fac64, *K64, prm.diag_quirk, 0.0, diag, nullptr, c.st);
   launch_max(diag, n, red(c, FIN_STORE, 1, nullptr, c.dscal + 0), kRedBlocks, c.st);
