@@ -74,16 +74,24 @@ struct BLevel {
   long long ndof = 0, nelem = 0;
   T *fac = nullptr, *xa = nullptr, *xb = nullptr, *b = nullptr, *r = nullptr;
   T* dn = nullptr;  // inverse diagonal per node of the smoothing instances
-  T *dinv = nullptr, *p = nullptr, *q = nullptr, *z = nullptr, *w = nullptr;  // coarse scratch
   DevTable smooth;   // instances that smooth here
-  DevTable coarse;   // instances whose coarsest level this is
   DevTable restr;    // next-level instances: g = next level, g2 = this level
   DevTable prolong;  // smoothing instances: g = this level, g2 = next level
+};
+
+// Coarsest-level solves of one launch: off and eoff of the table's entries
+// count from the bases below, off2 and noff from dinv, r, z, p, q and from w.
+template <typename T>
+struct BCoarse {
+  DevTable t;
+  T *fac = nullptr, *b = nullptr, *x = nullptr;  // level 0: b and x come with the call
+  T *dinv = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *w = nullptr;
 };
 
 template <typename T>
 struct BatchMG {
   std::vector<BLevel<T>> L;
+  BCoarse<T> c0, c1n;  // instances of one level; instances that end on levels >= 1
   ModalK<T> K;
   int quirk = 0, nu1 = 2, nu2 = 2, citers = 30;
   bool cheb = true, idx32 = true;
@@ -117,14 +125,23 @@ template <typename T>
 void bvcycle(BatchCtx& B, BatchMG<T>& mg, int l, const T* b, T* xout) {
   Ctx& c = B.c;
   BLevel<T>& V = mg.L[l];
-  if (V.coarse.n()) {
+  // The solves of instances that end on an earlier level wait for the deepest
+  // one: their CTAs run side by side there instead of one launch of a few CTAs
+  // per level (8 instances ending on three levels: 3 x 70 us a cycle -> 70).
+  // Nothing reads a level's correction before the way back up.
+  auto coarse = [&](const BCoarse<T>& S, const T* bb, T* x) {
+    if (!S.t.n()) return;
     long long mnd = 0, mne = 0;
-    for (const BatchInst& ci : V.coarse.h) mnd = std::max(mnd, ci.g.ndof()), mne = std::max(mne, ci.g.nelem());
-    launch_batch_coarse_pcg<T>(V.coarse.d, V.coarse.n(), V.fac, mg.K, V.dinv, b, xout, V.r, V.z, V.p, V.q, V.w,
-                               mg.citers, B.s, c.st, mnd, mne);
+    for (const BatchInst& ci : S.t.h) mnd = std::max(mnd, ci.g.ndof()), mne = std::max(mne, ci.g.nelem());
+    launch_batch_coarse_pcg<T>(S.t.d, S.t.n(), S.fac, mg.K, S.dinv, bb, x, S.r, S.z, S.p, S.q, S.w, mg.citers, B.s,
+                               c.st, mnd, mne);
     c.launches++;
+  };
+  if (l == 0) coarse(mg.c0, b, xout);
+  if (!V.smooth.n()) {
+    if (l > 0) coarse(mg.c1n, mg.c1n.b, mg.c1n.x);
+    return;
   }
-  if (!V.smooth.n()) return;
   const int nw = mg.nu1 + mg.nu2;
   auto bufw = [&](int w) -> T* { return ((nw - 1 - w) % 2 == 0) ? xout : V.xb; };
   int w = 0;
@@ -219,7 +236,12 @@ bool build_batch_mg(Ctx& c, BatchMG<T>& mg, const std::vector<Grid>& g0, const s
   int maxlev = 0;
   for (int v : nlev) maxlev = std::max(maxlev, v);
   mg.L.assign(maxlev, BLevel<T>());
+  mg.c0 = mg.c1n = BCoarse<T>();
   const std::string tag = sizeof(T) == 8 ? "bmg64_" : "bmg32_";
+  // the coarse levels' factors and vectors lie in one array each (levels start
+  // on multiples of 64 entries), so that one launch reaches all of them
+  std::vector<long long> loff(maxlev, 0), leoff(maxlev, 0);
+  long long cdof = 0, celem = 0;
   for (int l = 0; l < maxlev; ++l) {
     BLevel<T>& V = mg.L[l];
     for (int i = 0; i < n; ++i) {
@@ -234,14 +256,14 @@ bool build_batch_mg(Ctx& c, BatchMG<T>& mg, const std::vector<Grid>& g0, const s
       V.nelem += g.nelem();
     }
     const std::string s = tag + std::to_string(l);
-    V.fac = l == 0 ? const_cast<T*>(fac0) : c.vec<T>(s + "fac", V.nelem);
     V.xb = c.vec<T>(s + "xb", V.ndof);
     V.r = c.vec<T>(s + "r", V.ndof);
+    if (!V.xb || !V.r) return false;
     if (l > 0) {
-      V.xa = c.vec<T>(s + "xa", V.ndof);
-      V.b = c.vec<T>(s + "b", V.ndof);
+      loff[l] = cdof, leoff[l] = celem;
+      cdof += (V.ndof + 63) / 64 * 64;
+      celem += (V.nelem + 63) / 64 * 64;
     }
-    if (!V.fac || !V.xb || !V.r || (l > 0 && (!V.xa || !V.b))) return false;
     for (size_t k = 0; k < V.inst.size(); ++k) {
       const int i = V.inst[k];
       BatchInst bi;
@@ -254,7 +276,12 @@ bool build_batch_mg(Ctx& c, BatchMG<T>& mg, const std::vector<Grid>& g0, const s
       bi.sigma = sigma[i] * std::pow(8.0, l);  // row sums of P^T P
       bi.id = i;
       if (nlev[i] - 1 == l) {
-        V.coarse.h.push_back(bi);
+        BCoarse<T>& S = l == 0 ? mg.c0 : mg.c1n;
+        bi.off2 = S.t.n() ? S.t.h.back().off2 + S.t.h.back().g.ndof() : 0;
+        bi.noff = S.t.n() ? S.t.h.back().noff + S.t.h.back().g.nelem() : 0;
+        bi.off += loff[l];
+        bi.eoff += leoff[l];
+        S.t.h.push_back(bi);
       } else {
         V.smooth.h.push_back(bi);
         bi.g2 = batch_coarse_grid(bi.g);
@@ -262,14 +289,31 @@ bool build_batch_mg(Ctx& c, BatchMG<T>& mg, const std::vector<Grid>& g0, const s
         V.prolong.h.push_back(bi);  // off2 filled below
       }
     }
-    if (V.coarse.n()) {
-      V.dinv = c.vec<T>(s + "dinv", V.ndof);
-      V.p = c.vec<T>(s + "p", V.ndof);
-      V.q = c.vec<T>(s + "q", V.ndof);
-      V.z = c.vec<T>(s + "z", V.ndof);
-      V.w = c.vec<T>(s + "w", 24 * V.nelem);
-      if (!V.dinv || !V.p || !V.q || !V.z || !V.w) return false;
+  }
+  mg.c0.fac = mg.L[0].fac = const_cast<T*>(fac0);
+  if (maxlev > 1) {
+    mg.c1n.fac = c.vec<T>(tag + "fac", celem);
+    mg.c1n.x = c.vec<T>(tag + "xa", cdof);
+    mg.c1n.b = c.vec<T>(tag + "b", cdof);
+    if (!mg.c1n.fac || !mg.c1n.x || !mg.c1n.b) return false;
+    for (int l = 1; l < maxlev; ++l) {
+      mg.L[l].fac = mg.c1n.fac + leoff[l];
+      mg.L[l].xa = mg.c1n.x + loff[l];
+      mg.L[l].b = mg.c1n.b + loff[l];
     }
+  }
+  for (BCoarse<T>* S : {&mg.c0, &mg.c1n}) {
+    if (!S->t.n()) continue;
+    const std::string s = tag + (S == &mg.c0 ? "c0" : "c1");
+    const long long nd = S->t.h.back().off2 + S->t.h.back().g.ndof();
+    const long long nel = S->t.h.back().noff + S->t.h.back().g.nelem();
+    S->dinv = c.vec<T>(s + "dinv", nd);
+    S->r = c.vec<T>(s + "r", nd);
+    S->p = c.vec<T>(s + "p", nd);
+    S->q = c.vec<T>(s + "q", nd);
+    S->z = c.vec<T>(s + "z", nd);
+    S->w = c.vec<T>(s + "w", 24 * nel);
+    if (!S->dinv || !S->r || !S->p || !S->q || !S->z || !S->w || !upload(c, S->t, s + "tab")) return false;
   }
   for (int l = 0; l + 1 < maxlev; ++l) {
     BLevel<T>& V = mg.L[l];
@@ -306,8 +350,7 @@ bool build_batch_mg(Ctx& c, BatchMG<T>& mg, const std::vector<Grid>& g0, const s
     }
     if (V.restr.n()) V.restr.vblocks = vec_batch_plan(V.restr.h.data(), V.restr.n(), 1, kBatchVecBlocks);
     const std::string s = std::string(sizeof(T) == 8 ? "btab64_" : "btab32_") + std::to_string(l);
-    if (!upload(c, V.smooth, s + "s") || !upload(c, V.coarse, s + "c") || !upload(c, V.restr, s + "r") ||
-        !upload(c, V.prolong, s + "p"))
+    if (!upload(c, V.smooth, s + "s") || !upload(c, V.restr, s + "r") || !upload(c, V.prolong, s + "p"))
       return false;
     if (V.smooth.n() && node_dinv_ok(mg.K, mg.quirk)) {
       V.dn = c.vec<T>(tag + std::to_string(l) + "dn", V.ndof / 3);
@@ -318,11 +361,12 @@ bool build_batch_mg(Ctx& c, BatchMG<T>& mg, const std::vector<Grid>& g0, const s
         c.launches++;
       }
     }
-    for (const BatchInst& b : V.coarse.h) {
-      launch_diag<T>(b.g, b.m, V.fac + b.eoff, mg.K, mg.quirk, (T)b.sigma, nullptr, V.dinv + b.off, c.st);
+  }
+  for (const BCoarse<T>* S : {&mg.c0, &mg.c1n})
+    for (const BatchInst& b : S->t.h) {
+      launch_diag<T>(b.g, b.m, S->fac + b.eoff, mg.K, mg.quirk, (T)b.sigma, nullptr, S->dinv + b.off2, c.st);
       c.launches++;
     }
-  }
   mg.idx32 = true;
   for (const Grid& g : g0) mg.idx32 = mg.idx32 && g.ndof() < (1LL << 30) && g.nelem() < (1LL << 30);
   return true;

@@ -593,7 +593,9 @@ void launch_batch_jacobi0(const BatchInst* in, int ninst, int nblocks, const T* 
   batch_jacobi0_kernel<T><<<nblocks, 256, 0, st>>>(in, ninst, fac, K, quirk, omega, b, x, s);
 }
 
-// CTA i solves instance in[i] (vectors at off, element scratch w at 24 * eoff)
+// CTA i solves instance in[i]: factors at eoff, b and x at off, its inverse
+// diagonal and vectors at off2, its element scratch w at 24 * noff (a launch's
+// instances end on different levels, the scratch is theirs alone)
 template <typename T>
 __global__ void __launch_bounds__(1024) batch_coarse_pcg_kernel(const BatchInst* in, const T* __restrict__ fac,
                                                                 ModalK<T> K, const T* __restrict__ dinv,
@@ -601,9 +603,9 @@ __global__ void __launch_bounds__(1024) batch_coarse_pcg_kernel(const BatchInst*
                                                                 T* w, int iters, const PcgScalars* s) {
   const BatchInst& I = in[blockIdx.x];
   if (batch_halted(s, I.id)) return;
-  const long long o = I.off;
-  coarse_pcg_body<T>(I.g, I.m, fac + I.eoff, K, (T)I.sigma, dinv + o, b + o, x + o, r + o, z + o, p + o, q + o,
-                     w + 24 * I.eoff, iters);
+  const long long o = I.off2;
+  coarse_pcg_body<T>(I.g, I.m, fac + I.eoff, K, (T)I.sigma, dinv + o, b + I.off, x + I.off, r + o, z + o, p + o, q + o,
+                     w + 24 * I.noff, iters);
 }
 // The same Jacobi-PCG of one instance's coarsest grid with its five vectors
 // (x, r, z, p, q) and element factors held in shared memory, so every pass of
@@ -640,7 +642,7 @@ __global__ void __launch_bounds__(1024) batch_coarse_pcg_smem_kernel(const Batch
   T* sf = sq + n3;
   T* sw = sf + ne;  // W form only: 24 nElem words
   const T* gb = b + I.off;
-  const T* gd = dinv + I.off;
+  const T* gd = dinv + I.off2;
   const T* gf = fac + I.eoff;
   T part = T(0);
   for (int e = tid; e < ne; e += nthr) sf[e] = gf[e];
@@ -875,7 +877,7 @@ __global__ void __launch_bounds__(kRegThreads, 1)
     for (int c = 0; c < 3; ++c) {
       x[u][c] = 0.f;
       r[u][c] = t < nn ? b[I.off + 3 * t + c] : 0.f;
-      di[u][c] = t < nn ? dinv[I.off + 3 * t + c] : 0.f;
+      di[u][c] = t < nn ? dinv[I.off2 + 3 * t + c] : 0.f;
       p[u][c] = di[u][c] * r[u][c];
       part = fmaf(r[u][c], p[u][c], part);
     }
