@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(256) helm_update_kernel(Grid g, T* __restrict_
     acc[0] += rr;
     acc[1] += scale2(rr + (double)rz, on_face(j, g.NY) + on_face(k, g.NZ));
   }
-  block_reduce_finalize<2>(red, acc);
+  block_reduce_finalize<2, 256>(red, acc);
 }
 // One wave of warps with equal row counts (4 CTAs of 8 warps on each SM).
 static int helm_update_blocks(const Grid& g) {
@@ -426,7 +426,7 @@ __global__ void batch_helm_apply_kernel(const BatchInst* in, int ninst, HelmW<T>
   double acc[1] = {helm_apply_body<T>(I.g, W, x + I.noff, y + I.noff,
                                       (long long)(blockIdx.x - I.vblk0) * blockDim.x + threadIdx.x,
                                       (long long)I.vnblk * blockDim.x)};
-  block_reduce_finalize_at<1>(red, acc, I.id, blockIdx.x, I.vnblk, I.vblk0, 1);
+  block_reduce_finalize_at<1, 256>(red, acc, I.id, blockIdx.x, I.vnblk, I.vblk0, 1);
 }
 template <typename T>
 void launch_batch_helm_apply_dot(const BatchInst* in, int ninst, int nblocks, const HelmK& K, const T* x, T* y,

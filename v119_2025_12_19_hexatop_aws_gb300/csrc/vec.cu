@@ -308,7 +308,7 @@ __global__ void dot_kernel(const T* __restrict__ a, const T* __restrict__ b, con
     if (++cnt == kChunk) flush_parts<T, NS>(acc, part, cnt);
   }
   flush_parts<T, NS>(acc, part, cnt);
-  block_reduce_finalize<NS>(red, acc);
+  block_reduce_finalize<NS, 256>(red, acc);
 }
 template <typename T>
 void launch_dot(const T* a, const T* b, const T* c, const T* d, long long n, const RedArgs& red,
@@ -381,7 +381,7 @@ __global__ void pcg_update_kernel(T* __restrict__ x, T* __restrict__ r, T* __res
     if (++cnt == kChunk) flush_parts<T, NS>(acc, part, cnt);
   }
   flush_parts<T, NS>(acc, part, cnt);
-  block_reduce_finalize<NS>(red, acc);
+  block_reduce_finalize<NS, 256>(red, acc);
 }
 template <typename T>
 void launch_pcg_update(T* x, T* r, T* z, const T* p, const T* q, const T* dinv, long long n,
@@ -443,7 +443,7 @@ __global__ void pcg_update_mg_kernel(T* __restrict__ x, T* __restrict__ r, const
     if (++cnt == kChunk) flush_parts<T, 2>(acc, part, cnt);
   }
   flush_parts<T, 2>(acc, part, cnt);
-  block_reduce_finalize<2>(red, acc);
+  block_reduce_finalize<2, 256>(red, acc);
 }
 template <typename T>
 void launch_pcg_update_mg(T* x, T* r, const T* p, const T* q, const T* zo, long long n, const RedArgs& red,
@@ -500,7 +500,7 @@ __global__ void jacobi_precond_kernel(T* __restrict__ z, const T* __restrict__ r
     if (++cnt == kChunk) flush_parts<T, 1>(acc, part, cnt);
   }
   flush_parts<T, 1>(acc, part, cnt);
-  block_reduce_finalize<1>(red, acc);
+  block_reduce_finalize<1, 256>(red, acc);
 }
 template <typename T>
 void launch_jacobi_precond(T* z, const T* r, const T* dinv, long long n, const RedArgs& red,
@@ -633,7 +633,7 @@ __global__ void batch_pcg_update_kernel(const BatchInst* in, int ninst, int node
     if (++cnt == kChunk) flush_parts<T, NS>(acc, part, cnt);
   }
   flush_parts<T, NS>(acc, part, cnt);
-  block_reduce_finalize_at<NS>(red, acc, sg.id, blockIdx.x, sg.nblk, sg.blk0, 1);
+  block_reduce_finalize_at<NS, 256>(red, acc, sg.id, blockIdx.x, sg.nblk, sg.blk0, 1);
 }
 template <typename T>
 void launch_batch_pcg_update(const BatchInst* in, int ninst, int nblocks, int node_sized, T* x, T* r, T* z,
@@ -675,7 +675,7 @@ __global__ void batch_dot_kernel(const BatchInst* in, int ninst, int node_sized,
     if (++cnt == kChunk) flush_parts<T, NS>(acc, part, cnt);
   }
   flush_parts<T, NS>(acc, part, cnt);
-  block_reduce_finalize_at<NS>(red, acc, sg.id, blockIdx.x, sg.nblk, sg.blk0, 1);
+  block_reduce_finalize_at<NS, 256>(red, acc, sg.id, blockIdx.x, sg.nblk, sg.blk0, 1);
 }
 template <typename T>
 void launch_batch_dot(const BatchInst* in, int ninst, int nblocks, int node_sized, const T* a, const T* b,
