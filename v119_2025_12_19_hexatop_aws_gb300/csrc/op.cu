@@ -654,7 +654,7 @@ __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, in
   // x, b and the previous iterate two layers past the register prefetch, into
   // L2: 384x192x192 Chebyshev step 0.2207 -> 0.2160 ms, residual 0.2086 ->
   // 0.2032, apply with p.Ap 0.2022 -> 0.1978; three to six layers gain less.
-  // Only in the kernels of grids whose vectors overflow L2 (launch_op).
+  // Only in the kernels of grids whose vectors overflow L2 (see launch_op).
   const IX touch0 = (IX)3 * ((IX)min(in, g.NX - 1) + (IX)g.NX * min(jn, g.NY - 1));
   auto touch_l2 = [&](int k) {
     if (!TOUCH || k + 3 >= k1) return;
@@ -1475,12 +1475,14 @@ void launch_op(int mode, const OpArgs<T>& a0, cudaStream_t st) {
     }
     return;
   }
-  // FP32 vectors of which one overflows L2 are prefetched into it ahead of the
-  // march: 2 to 3% of a launch at 384x192x192 (172 MB a vector); at 192^3 (86 MB)
-  // the same prefetch cost a multigrid solve 2% (91.3 -> 93.6 ms), its
-  // instructions alone, switched off at run time, 1.8%.
+  // Prefetch into L2 ahead of the march where three FP32 vectors overflow it
+  // (126 MB) and so do not stay there between launches:
+  // Chebyshev step without / with it 30.9 / 32.9 us at 192x96x96 (22 MB a
+  // vector; a multigrid solve lost 2%), 79.8 / 78.0 at 256x128x128 (51 MB),
+  // 130.5 / 126.9 at 320x160x160, 221 / 215 at 384x192x192.  A form of its own:
+  // the instructions alone, switched off at run time, cost the small grid 1.8%.
   constexpr bool F32 = sizeof(T) == 4;
-  const bool touch = F32 && a.g.ndof() * (long long)sizeof(T) > (120LL << 20);
+  const bool touch = F32 && a.g.ndof() * (long long)sizeof(T) > (40LL << 20);
 #define HEXA_OP_CASE(M)                                                              \
   case M:                                                                           \
     if (i32 && touch) op_kernel<T, M, TYW, int, false, F32><<<grid, block, 0, st>>>(a);  \
