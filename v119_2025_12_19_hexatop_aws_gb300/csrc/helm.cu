@@ -125,6 +125,8 @@ HelmPlan helm_plan(const Grid& g) {
       if (c < cost) {
         cost = c;
         best.tx = tx, best.ty = ty, best.threads = thr, best.ntx = (int)nx, best.nty = (int)ny;
+        // whole warps with 2 * stage >= nodes (rounded up before the halving: a 53 x 5 tile has an odd 385)
+        best.stage = (((tx + 2) * (ty + 2) + 1) / 2 + 31) / 32 * 32;
       }
     }
   const long long tiles = (long long)best.ntx * best.nty;
@@ -164,7 +166,7 @@ __global__ void __launch_bounds__(288, 3) helm_dir_kernel(Grid g, HelmPlan pl, H
   const int tiles = pl.ntx * pl.nty;
   const long long plane = (long long)g.NX * g.NY;
   // the first warps stage two nodes per thread, the others none
-  const int half = (nslots / 2 + 31) / 32 * 32;
+  const int half = pl.stage;
   const bool stager = tid < half;
   const bool two = stager && tid + half < nslots;
   const int lx = tid % pl.tx, ly = tid / pl.tx, c = (lx + 1) + SX * (ly + 1);

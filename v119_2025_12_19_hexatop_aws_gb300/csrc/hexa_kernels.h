@@ -163,6 +163,7 @@ void launch_helm_init(const Grid& g, const HelmK& K, const TI* rho, T* r, const 
 // pn = z + beta po, q = A pn, sum pn.q (po and pn are different vectors)
 struct HelmPlan {
   int tx, ty, threads;  // columns of a tile, threads of a CTA
+  int stage;            // threads that stage the tile and its halo, two nodes each
   int ntx, nty, kchunk; // tiles per axis, layers per item
   long long items;
   int blocks;
