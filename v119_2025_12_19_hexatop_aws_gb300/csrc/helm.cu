@@ -81,12 +81,15 @@ static HelmW<T> helm_weights(const HelmK& K) {
 __device__ __forceinline__ int on_face(int i, int n) { return (i == 0) | (i == n - 1); }
 // v * 2^faces (-3 <= faces <= 3): a node on `faces` (0..3) faces of the box has 2^-faces of the
 // inner nodes' diagonal.  Through the exponent bits, so that nothing is issued
-// to the FP64 pipe (zero, subnormal and non-finite values stay as they are; no
-// value here is near the upper end of the range).
+// to the FP64 pipe.  Values whose exponent field could leave its range stay as
+// they are: zeros and magnitudes below 2^-1019, which are nothing beside
+// the terms they are added to, and non-finite values and magnitudes from 2^1021,
+// whose squares have overflowed the PCG's sums anyway.
 __device__ __forceinline__ float scale2(float v, int faces) { return v * __int_as_float((127 + faces) << 23); }
 __device__ __forceinline__ double scale2(double v, int faces) {
-  const int hi = __double2hiint(v), e = hi & 0x7ff00000;
-  return __hiloint2double(hi + ((e == 0 || e == 0x7ff00000) ? 0 : faces * (1 << 20)), __double2loint(v));
+  const int hi = __double2hiint(v);
+  const bool in = (unsigned)(hi & 0x7ff00000) - 0x00400000u < 0x7f800000u;  // exponent field 4 .. 0x7fb
+  return __hiloint2double(hi + (in ? faces * (1 << 20) : 0), __double2loint(v));
 }
 
 // ---- one grid: the PCG in two launches per iteration
