@@ -55,6 +55,9 @@ long long op_num_blocks(const Grid& g, int kchunk);
 // node layers per work item of a mode's launches (see op.cu)
 template <typename T>
 int op_pick_kchunk(const Grid& g, int mode = OP_APPLY);
+// the rule behind it: layers per chunk for `tiles` columns of NZ layers on
+// `ctas` resident CTAs, an item costing `start` layers besides its own
+int op_chunk_layers(long long tiles, int NZ, long long ctas, double start);
 ModalK<float> modal_to_f32(const ModalK<double>& K);
 
 // ------------------------------------------------------------ vector passes

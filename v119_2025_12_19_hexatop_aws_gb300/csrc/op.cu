@@ -1339,6 +1339,21 @@ constexpr double op_item_start() { return sizeof(T) == 8 ? 0.6 : 2.0; }
 // layers and fill the SMs (a 24x12x12 grid is one tile: one CTA marching its 13
 // layers took 13.6 us, 13 CTAs of one layer 5 us); large ones keep long
 // chunks that divide evenly over the CTAs.
+// Tried up to four items a CTA, and up to 64 chunks where there are more tiles
+// than that: a slender column (one tile, 2001 layers) takes one chunk per CTA.
+int op_chunk_layers(long long tiles, int NZ, long long ctas, double start) {
+  const int most = (int)std::min<long long>(NZ, std::max<long long>(64, 4 * ctas / tiles));
+  double best = 1e300;
+  int kbest = NZ;
+  for (int n = 1; n <= most; ++n) {
+    const int kc = (NZ + n - 1) / n;
+    const long long items = tiles * ((NZ + kc - 1) / kc);
+    const double t = (double)((items + ctas - 1) / ctas) * (kc + start);
+    if (t < best) best = t, kbest = kc;
+  }
+  return kbest;
+}
+
 template <typename T>
 int op_pick_kchunk(const Grid& g, int mode) {
   int tx, ty, nch;
@@ -1350,15 +1365,7 @@ int op_pick_kchunk(const Grid& g, int mode) {
     chunks = std::max<long long>(1, std::min<long long>(chunks, (g.NZ + 15) / 16));
     return (int)((g.NZ + chunks - 1) / chunks);
   }
-  double best = 1e300;
-  int kbest = g.NZ;
-  for (int n = 1; n <= std::min(g.NZ, 64); ++n) {
-    const int kc = (g.NZ + n - 1) / n;
-    const long long items = tiles * ((g.NZ + kc - 1) / kc);
-    const double t = (double)((items + ctas - 1) / ctas) * (kc + op_item_start<T>());
-    if (t < best) best = t, kbest = kc;
-  }
-  return kbest;
+  return op_chunk_layers(tiles, g.NZ, ctas, op_item_start<T>());
 }
 
 static int tma_resident_ctas() {
