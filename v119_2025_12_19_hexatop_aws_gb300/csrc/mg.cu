@@ -970,35 +970,29 @@ size_t batch_coarse_smem_bytes(long long max_ndof, long long max_nelem, bool scr
   return bytes <= 220u * 1024u ? bytes : 0;
 }
 
+// The shared-memory limits are a device's: set before each launch (a few per
+// solve, captured into its graph), for the contexts of every device.
 template <typename T>
 void launch_batch_coarse_pcg(const BatchInst* in, int ninst, const T* fac, const ModalK<T>& K, const T* dinv,
                              const T* b, T* x, T* r, T* z, T* p, T* q, T* w, int iters, const PcgScalars* s,
                              cudaStream_t st, long long max_ndof, long long max_nelem) {
   if constexpr (sizeof(T) == 4) {
     if (max_ndof <= 3 * kRegMax && max_nelem <= kRegMax) {
-      static bool attr_reg = false;
-      if (!attr_reg) {
-        cudaFuncSetAttribute(batch_coarse_pcg_reg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(CoarseRegSmem));
-        attr_reg = true;
-      }
+      cudaFuncSetAttribute(batch_coarse_pcg_reg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(CoarseRegSmem));
       batch_coarse_pcg_reg_kernel<<<ninst, kRegThreads, sizeof(CoarseRegSmem), st>>>(in, fac, K, dinv, b, x, iters, s);
       return;
     }
   }
   const size_t smem_w = batch_coarse_smem_bytes<T>(max_ndof, max_nelem, true);
   const size_t smem_c = batch_coarse_smem_bytes<T>(max_ndof, max_nelem, false);
-  static bool attr = false;
-  if (!attr && smem_c > 0) {
-    cudaFuncSetAttribute(batch_coarse_pcg_smem_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(batch_coarse_pcg_smem_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    attr = true;
-  }
   if (smem_w > 0) {
+    cudaFuncSetAttribute(batch_coarse_pcg_smem_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     batch_coarse_pcg_smem_kernel<T, true><<<ninst, 1024, smem_w, st>>>(in, fac, K, dinv, b, x, iters, s);
     return;
   }
   if (smem_c > 0) {
+    cudaFuncSetAttribute(batch_coarse_pcg_smem_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     batch_coarse_pcg_smem_kernel<T, false><<<ninst, 1024, smem_c, st>>>(in, fac, K, dinv, b, x, iters, s);
     return;
   }
