@@ -62,18 +62,32 @@ void stage_out(Ctx& c, T* user, const T* dev, size_t n) {
   if (user != dev) cudaMemcpyAsync(user, dev, n * sizeof(T), cudaMemcpyDeviceToHost, c.st);
 }
 
-// Per-node fixed bits from a per-DOF byte mask (host or device), packed on the
-// device: a host pass over the mask took 1.3 ms of a 1.4 ms product on
-// 190x93x61 elements.
-const uint8_t* node_mask(Ctx& c, const Grid& g, const uint8_t* fixed_dof) {
-  if (!fixed_dof) return nullptr;
+// Mask of the boundary conditions: the clamped faces and, from a per-DOF byte
+// mask (host or device), bits per node, packed on the device: a host pass over
+// the mask took 1.3 ms of a 1.4 ms product on 190x93x61 elements.  A solve drops
+// a mask that fixes nothing, which all its kernels would read; a single launch
+// reads it (1 B a node) rather than wait for the answer.  False when the
+// mask's buffers cannot be had.
+bool make_mask(Ctx& c, const Grid& g, const hexa_bc* bc, bool drop_empty, Mask* m) {
+  m->faces = bc ? bc->clamp_faces : 0u;
+  m->node = nullptr;
+  if (!bc || !bc->fixed_dof) return true;
   const long long nn = g.nnode();
-  const uint8_t* f = stage_in<uint8_t>(c, fixed_dof, 3 * nn, "nodemask_dof");
+  const uint8_t* f = stage_in<uint8_t>(c, bc->fixed_dof, 3 * nn, "nodemask_dof");
   uint8_t* d = c.vec<uint8_t>("nodemask", nn);
-  if (!f || !d) return nullptr;
-  launch_node_bits(f, d, nn, c.st);
+  int* any = drop_empty ? c.vec<int>("nodemask_any", 1) : nullptr;
+  if (!f || !d || (drop_empty && !any)) return false;
+  if (any) cudaMemsetAsync(any, 0, sizeof(int), c.st);
+  launch_node_bits(f, d, any, nn, c.st);
   c.launches++;
-  return d;
+  if (any) {
+    int h = 0;
+    cudaMemcpyAsync(&h, any, sizeof(int), cudaMemcpyDeviceToHost, c.st);
+    if (cudaStreamSynchronize(c.st) != cudaSuccess) return c.cuda_ok("mask");
+    if (!h) return true;
+  }
+  m->node = d;
+  return true;
 }
 
 // build_modal through the context's cache of the last geometry.
@@ -97,9 +111,7 @@ bool prepare_problem(hexa_ctx* h, const hexa_grid* g, const hexa_bc* bc, double 
   P->dy = g->dy;
   P->dz = g->dz;
   P->nu = nu;
-  P->m.faces = bc ? bc->clamp_faces : 0u;
-  P->m.node = bc ? node_mask(c, P->g, bc->fixed_dof) : nullptr;
-  if (bc && bc->fixed_dof && !c.err.empty()) return false;
+  if (!make_mask(c, P->g, bc, true, &P->m)) return false;
   P->fac64 = stage_in<double>(c, factor, P->g.nelem(), "in_factor");
   if (!P->fac64) return false;
   if (f) {
@@ -261,8 +273,7 @@ static int apply_operator_t(hexa_ctx* h, const hexa_grid* g, const hexa_bc* bc, 
   if (!modal_of(c, g, nu, &K64, &e)) return set_err(h, HEXA_ERR_ARG, e);
   const Grid G = make_grid(g->nx, g->ny, g->nz);
   Mask m;
-  m.faces = bc ? bc->clamp_faces : 0u;
-  m.node = bc ? node_mask(c, G, bc->fixed_dof) : nullptr;
+  if (!make_mask(c, G, bc, false, &m)) return HEXA_ERR_NOMEM;
   const T* fac = stage_in<T>(c, factor, G.nelem(), sizeof(T) == 8 ? "ap_fac64" : "ap_fac32");
   const T* xr = stage_in<T>(c, x, G.ndof(), sizeof(T) == 8 ? "ap_xr64" : "ap_xr32");
   T* yd = out_buf<T>(c, y, G.ndof(), sizeof(T) == 8 ? "ap_y64" : "ap_y32");
@@ -341,8 +352,7 @@ static int time_operator_t(hexa_ctx* h, const hexa_grid* g, const hexa_bc* bc, d
   if ((mode == OP_RESID || mode == OP_JACOBI || mode == OP_CHEB2) && !b) return set_err(h, HEXA_ERR_ARG, "mode needs b");
   const Grid G = make_grid(g->nx, g->ny, g->nz);
   Mask m;
-  m.faces = bc ? bc->clamp_faces : 0u;
-  m.node = bc ? node_mask(c, G, bc->fixed_dof) : nullptr;
+  if (!make_mask(c, G, bc, false, &m)) return HEXA_ERR_NOMEM;
   OpArgs<T> a;
   a.g = G;
   a.m = m;
@@ -414,8 +424,7 @@ int hexa_operator_diagonal(hexa_ctx* h, const hexa_grid* g, const hexa_bc* bc, d
   if (!modal_of(c, g, nu, &K64, &e)) return set_err(h, HEXA_ERR_ARG, e);
   const Grid G = make_grid(g->nx, g->ny, g->nz);
   Mask m;
-  m.faces = bc ? bc->clamp_faces : 0u;
-  m.node = bc ? node_mask(c, G, bc->fixed_dof) : nullptr;
+  if (!make_mask(c, G, bc, false, &m)) return HEXA_ERR_NOMEM;
   const double* fac = stage_in<double>(c, factor, G.nelem(), "ap_fac64");
   double* d = out_buf<double>(c, diag_out, G.ndof(), "ap_y64");
   if (!fac || !d) return HEXA_ERR_NOMEM;

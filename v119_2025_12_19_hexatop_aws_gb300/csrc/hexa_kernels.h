@@ -72,8 +72,8 @@ void launch_copy(T* dst, const T* src, long long n, cudaStream_t st);
 // dst = src with fixed DOFs zeroed (expand/contract semantics)
 template <typename TD, typename TS>
 void launch_mask_copy(const Grid& g, const Mask& m, TD* dst, const TS* src, cudaStream_t st);
-// Per-node bits (bit c: component c fixed) from one byte per DOF
-void launch_node_bits(const uint8_t* fixed_dof, uint8_t* bits, long long nnode, cudaStream_t st);
+// Per-node bits (bit c: component c fixed) from one byte per DOF; *any (nullable) |= any bit set
+void launch_node_bits(const uint8_t* fixed_dof, uint8_t* bits, int* any, long long nnode, cudaStream_t st);
 // Jacobi inverse diagonal dinv = 1/(dd*fsum + sigma) (0 at fixed DOFs) and
 // the raw diagonal (dd*fsum, 0 at fixed DOFs).
 template <typename T>

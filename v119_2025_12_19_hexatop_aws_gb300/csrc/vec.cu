@@ -111,12 +111,17 @@ void launch_mask_copy(const Grid& g, const Mask& m, TD* dst, const TS* src, cuda
 }
 
 // A warp's 32 nodes are 96 mask bytes: three coalesced byte loads per thread.
-__global__ void node_bits_kernel(const uint8_t* __restrict__ fixed, uint8_t* __restrict__ bits, long long nn) {
-  for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nn; n += (long long)gridDim.x * blockDim.x)
-    bits[n] = (uint8_t)((fixed[3 * n] ? 1 : 0) | (fixed[3 * n + 1] ? 2 : 0) | (fixed[3 * n + 2] ? 4 : 0));
+__global__ void node_bits_kernel(const uint8_t* __restrict__ fixed, uint8_t* __restrict__ bits, int* any, long long nn) {
+  bool set = false;
+  for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nn; n += (long long)gridDim.x * blockDim.x) {
+    const uint8_t b = (uint8_t)((fixed[3 * n] ? 1 : 0) | (fixed[3 * n + 1] ? 2 : 0) | (fixed[3 * n + 2] ? 4 : 0));
+    bits[n] = b;
+    set |= b != 0;
+  }
+  if (any && set) *any = 1;
 }
-void launch_node_bits(const uint8_t* fixed_dof, uint8_t* bits, long long nnode, cudaStream_t st) {
-  node_bits_kernel<<<vec_blocks(nnode), 256, 0, st>>>(fixed_dof, bits, nnode);
+void launch_node_bits(const uint8_t* fixed_dof, uint8_t* bits, int* any, long long nnode, cudaStream_t st) {
+  node_bits_kernel<<<vec_blocks(nnode), 256, 0, st>>>(fixed_dof, bits, any, nnode);
 }
 
 // Sum of the factors of the (up to) 8 elements around node (i,j,k).
