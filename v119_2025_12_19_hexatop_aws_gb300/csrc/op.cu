@@ -292,30 +292,51 @@ __device__ __forceinline__ void element_modal<float>(const ModalK<float>& K, con
 // ------------------------------------------ FP64 element product in integers
 // The FP64 operator is bound by FP64 issue: 2 instructions per clock and SM,
 // against 64 or more integer ones.  An element's product is therefore formed in
-// 64-bit fixed point, scaled per element, and only the sums over elements (with
-// the factors) stay FP64: 36 FP64 instructions an element layer instead of 190.
-//   * a node layer's corner values become integers at the layer's largest
-//     exponent (58 bits; FP64's 53 are exact down to 2^-5 of the largest), and
-//     the butterflies on them are exact;
-//   * the strain modes are normalised by a common shift (61 bits), so the
+// 64-bit fixed point, and only the sums over elements (with the factors) stay
+// FP64: 36 FP64 instructions an element layer instead of 190.
+//   * each component of a node layer's corner values becomes integers at the
+//     component's own largest exponent (58 bits; FP64's 53 are exact down to
+//     2^-5 of the largest), and the butterflies on them are exact: a rigid
+//     translation drops out without a trace;
+//   * the strain modes are normalised by their largest (60 bits), so the
 //     precision follows the strains, not the rigid motion they were taken from;
 //   * the modal blocks multiply as two 32-bit halves (vh ch, vh cl, vl ch
-//     accumulated in 64 bits; the dropped vl cl is below 2^-60 of the largest
-//     mode times the largest coefficient), the inverse butterflies are exact.
-// Each rounding is relative to the element's largest mode and below 2^-58 of
-// it, where FP64 rounds at 2^-53 of every intermediate sum.  Chosen when the
-// smallest non-zero modal coefficient is within 2^-6 of the largest (every brick
-// and nu in ordinary use; not nu near 0.5 or needle elements), else the FP64
-// form.  The norm of the true residual (OP_RESID_NORM), which a solve reports,
-// stays in the FP64 form: a caller who recomputes it in FP64 at the rounding
-// limit finds that arithmetic's rounding in it (single solves, batches).  A
-// non-finite corner makes the element's product NaN.
-// 256x128x128 product: 0.60 ms, 1.90 in FP64 (8 warps and 0.82 ms with the
-// layers prefetched into registers; 14 and 16 warps 0.63 and 0.64); against
-// quad precision its error is 0.90 to 1.00 of the FP64 form's on random
-// displacements and 0.04 to 0.4 on smooth ones, where FP64 loses the strains to
-// the rigid motion.
+//     accumulated in 64 bits and rounded; the dropped vl cl is below 2^-58 of the
+//     largest mode times the largest coefficient), the inverse butterflies are
+//     exact.
+// The modes that enter one component's forces can be far smaller than others
+// that do not (a force in x feels four of the seven modes of u_z).  Where
+// they are within 2^-3 of the largest, for each component, one
+// scale serves the element; elsewhere (kFixedGap) each of the eleven sub-blocks
+// that couple has its own, and each component's sums are aligned to the largest term
+// that they have.  So a rounding is below about 2^-55 of the largest term of the
+// force component that it enters, where FP64 rounds at 2^-53 of every
+// intermediate sum.
+// Chosen when the smallest modal coefficient is within 2^-6 of the largest
+// (bricks and nu in ordinary use; not nu = 0, nu near 0.5 or needle elements),
+// else the FP64 form.  The norm of the true residual (OP_RESID_NORM), which a
+// solve reports, stays in the FP64 form: a caller who recomputes it in FP64 at
+// the rounding limit finds that arithmetic's rounding in it (single solves,
+// batches).  A non-finite corner makes the element's product NaN.
+// 256x128x128 product: 0.65 ms on random displacements and 0.69 on a bending field,
+// 1.90 in FP64 (0.63 and 0.64 with one exponent for the three components, whose
+// error in a small component beside a large one has no bound; 0.66 and 0.75 on random
+// displacements with the general form inlined and with it alone).
+// Against quad precision the error, per component, is 0.94 to 1.00 of the FP64
+// form's on random displacements, 0.06 to 0.6 on smooth ones, and 0.9 to 1.3
+// (at 2e-16) where FP64 is exact but for its last sums: constants and 0/1
+// patterns in one component beside values down to 1e-12 of it in the others.
 constexpr int kFixedWarps = 12;  // one CTA per SM at 168 registers
+// Sub-block s: class q and the components that it couples.  Classes 0 and 7
+// couple all three; a one-bit class the two components other than its
+// bit's; a two-bit class those two and, alone, the third.
+constexpr int kSub = 11;
+__host__ __device__ constexpr int sub_q(int s) { return s < 2 ? 7 * s : s < 5 ? 1 << (s - 2) : 7 ^ (1 << ((s - 5) % 3)); }
+__host__ __device__ constexpr bool sub_has(int s, int c) {
+  return s < 2 ? true : s < 8 ? c != (s - 2) % 3 : c == s - 8;
+}
+constexpr int kNoMode = -100000;  // the exponent of nothing
+constexpr int kFixedGap = 3;  // 2: 0.80 ms on the bending field; 4: errors above FP64's on sparse modes
 struct FixedK {
   int h[8][3][3], l[8][3][3];  // B = (h 2^32 + l) 2^-exp, l signed
   int exp;
@@ -330,62 +351,56 @@ static FixedK fixed_blocks(const ModalK<double>& K) {
         if (modal_nz(q, c, d)) {
           const double v = std::fabs(K.B[q][c][d]);
           mx = std::max(mx, v);
+          mn = std::min(mn, v);
         }
-  for (int q = 0; q < 8; ++q)
-    for (int c = 0; c < 3; ++c)
-      for (int d = 0; d < 3; ++d) {
-        const double v = std::fabs(K.B[q][c][d]);
-        if (v > 1e-12 * mx) mn = std::min(mn, v);  // below: zero but for the quadrature's rounding
-      }
   F.ok = std::isfinite(mx) && mx > 0.0 && mn >= mx / 64.0;
   int e = 0;
-  std::frexp(mx, &e);  // mx < 2^e
+  if (F.ok) std::frexp(mx, &e);  // mx < 2^e
   F.exp = 61 - e;
   for (int q = 0; q < 8; ++q)
     for (int c = 0; c < 3; ++c)
       for (int d = 0; d < 3; ++d) {
-        const long long v = F.ok ? std::llrint(std::ldexp(K.B[q][c][d], F.exp)) : 0;
+        const long long v = F.ok && modal_nz(q, c, d) ? std::llrint(std::ldexp(K.B[q][c][d], F.exp)) : 0;
         F.l[q][c][d] = (int)(v & 0xffffffffLL);
         F.h[q][c][d] = (int)((v - F.l[q][c][d]) >> 32);
       }
   return F;
 }
 
-// Corner values -> xy-modal integers; returns the layer's exponent field (the
-// integers are in units of 2^(E - 1080)), 0x7ff when a value is not finite.
-__device__ __forceinline__ int fixed_layer(const double (&v)[4][3], long long (&m)[4][3]) {
-  unsigned mx = 0;
-#pragma unroll
-  for (int cc = 0; cc < 4; ++cc)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) mx = max(mx, (unsigned)__double2hiint(v[cc][c]) & 0x7fffffffu);
-  const int E = (int)(mx >> 20);
+// Corner values -> xy-modal integers and the components' exponent fields (the
+// integers are in units of 2^(E - 1080)), 0x7ff where a value is not finite.
+__device__ __forceinline__ void fixed_layer(const double (&v)[4][3], long long (&m)[4][3], int (&E)[3]) {
   long long q[4][3];
 #pragma unroll
-  for (int cc = 0; cc < 4; ++cc)
+  for (int c = 0; c < 3; ++c) {
+    unsigned mx = 0x100000u;  // subnormal values have the smallest normal ones' exponent
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
+    for (int cc = 0; cc < 4; ++cc) mx = max(mx, (unsigned)__double2hiint(v[cc][c]) & 0x7fffffffu);
+    E[c] = (int)(mx >> 20);
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) {
       const int hi = __double2hiint(v[cc][c]);
-      const int e = (hi >> 20) & 0x7ff;
+      const unsigned a = (unsigned)hi & 0x7fffffffu;
+      const int e = max((int)(a >> 20), 1);
       const unsigned long long mant =
-          ((unsigned long long)(unsigned)((hi & 0xfffff) | 0x100000) << 32 | (unsigned)__double2loint(v[cc][c])) << 5;
-      const int d = e == 0 ? 63 : min(E - e, 63);  // zero and subnormal values: 0
-      q[cc][c] = (long long)(mant >> d) ^ (long long)(hi >> 31);  // negative: one's complement, one unit below
+          ((unsigned long long)(a - ((unsigned)(e - 1) << 20)) << 32 | (unsigned)__double2loint(v[cc][c])) << 5;
+      const long long x = (long long)(mant >> min(E[c] - e, 63));
+      q[cc][c] = hi < 0 ? -x : x;
     }
+  }
   xy_forward<long long>(q, m);
-  return E;
 }
 
-// q rounded to a double, by integer operations: the conversion instruction runs
-// on the FP64 pipe (0.80 ms against 0.60 for the 256x128x128 product).  The
-// leading bit is looked for in the high word; values below 2^32 units shift
-// their low word up.  A carry out of the mantissa runs into the exponent.
-__device__ __forceinline__ double fixed_to_double(long long q) {
+// q 2^(ex - 1085) rounded to a double, by integer operations: the conversion
+// instruction runs on the FP64 pipe (0.80 ms against 0.63 for the 256x128x128
+// product).  The leading bit is looked for in the high word; values below 2^32
+// units shift their low word up.  A carry out of the mantissa runs into the
+// exponent.
+__device__ __forceinline__ double fixed_to_double(long long q, int ex) {
   const unsigned s = (unsigned)((int)(q >> 32) >> 31);
   unsigned uh = (unsigned)(q >> 32) ^ s, ul = (unsigned)q ^ s;
-  int ex = 1085;
   if (uh == 0) {
-    uh = ul, ul = 0, ex = 1053;
+    uh = ul, ul = 0, ex -= 32;
     if (uh == 0) return 0.0;
   }
   const int z = __clz((int)uh);
@@ -396,80 +411,193 @@ __device__ __forceinline__ double fixed_to_double(long long q) {
                           (int)(unsigned)b);
 }
 
-// f * 2^x
-__device__ __forceinline__ double scale_exp(double f, int x) {
+// f * 2^x = the returned value * 2^(ex - 1085), ex for fixed_to_double: where
+// f * 2^x itself would lose bits below the normal numbers, the integers take 2^-512.
+__device__ __forceinline__ double scale_exp(double f, int x, int* ex) {
   const int hi = __double2hiint(f), e = (hi >> 20) & 0x7ff;
-  if (e != 0 && e != 0x7ff && e + x > 0 && e + x < 0x7ff)
-    return __hiloint2double(hi + x * (1 << 20), __double2loint(f));
+  *ex = 1085;
+  if (e != 0 && e != 0x7ff && e + x > 128 && e + x < 0x7ff) return __hiloint2double(hi + x * (1 << 20), __double2loint(f));
+  if (e + x <= 128) *ex = 1085 - 512, x += 512;
   return scalbn(f, x);  // zero, subnormal, non-finite or out of range
 }
 
+// Exponent of a mode: its leading bit and its component's; kNoMode for 0.
+__device__ __forceinline__ int mode_top(long long t, int E) {
+  const int hi = (int)(t >> 32), lo = (int)t, s = hi >> 31;
+  const int a = hi ^ s, b = lo ^ s;
+  const int z = a ? __clz(a) : 32 + __clz(b);
+  return (hi | lo) ? E - z : kNoMode;
+}
+
+// One sub-block on normalised modes, in place.
+template <int SUB>
+__device__ __forceinline__ void fixed_product(const FixedK& K, long long (&h)[8][3]) {
+  constexpr int q = sub_q(SUB);
+  int vh[3], vl[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    if (sub_has(SUB, c)) {
+      const long long t = h[q ^ (1 << c)][c];
+      vl[c] = (int)t;
+      vh[c] = (int)(t >> 32) - (vl[c] >> 31);
+    }
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    if (sub_has(SUB, c)) {
+      long long A = 0, M = 1LL << 31;
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (sub_has(SUB, d)) {
+          A += (long long)vh[d] * K.h[q][c][d];
+          M += (long long)vh[d] * K.l[q][c][d];
+          M += (long long)vl[d] * K.h[q][c][d];
+        }
+      h[q ^ (1 << c)][c] = A + (M >> 32);
+    }
+}
+template <int SUB>
+__device__ __forceinline__ void fixed_sub_blocks(const FixedK& K, const int (&E)[3], long long (&h)[8][3],
+                                                 int (&S)[kSub], int (&T)[3]) {
+  if constexpr (SUB < kSub) {
+    constexpr int q = sub_q(SUB);
+    int S0 = kNoMode;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      if (sub_has(SUB, c)) S0 = max(S0, mode_top(h[q ^ (1 << c)][c], E[c]));
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      if (sub_has(SUB, c)) {  // the largest mode to 60 bits
+        const int k = E[c] - S0 - 3;
+        long long& t = h[q ^ (1 << c)][c];
+        t = (t << min(max(k, 0), 63)) >> min(max(-k, 0), 63);
+        T[c] = max(T[c], S0);
+      }
+    S[SUB] = S0;
+    fixed_product<SUB>(K, h);
+    fixed_sub_blocks<SUB + 1>(K, E, h, S, T);
+  }
+}
+template <int SUB>
+__device__ __forceinline__ void fixed_products(const FixedK& K, long long (&h)[8][3]) {
+  if constexpr (SUB < kSub) {
+    fixed_product<SUB>(K, h);
+    fixed_products<SUB + 1>(K, h);
+  }
+}
+
+// The general form of the normalisation and the product, a function of its own so that
+// its registers are not the common path's (h: 8 x 3 modes in, products out).
+__device__ __noinline__ void fixed_general(const FixedK& K, long long* hm, int E0, int E1, int E2, int* Tm) {
+  long long h[8][3];
+  const int E[3] = {E0, E1, E2};
+  int S[kSub], T[3] = {kNoMode, kNoMode, kNoMode};
+#pragma unroll
+  for (int m = 0; m < 8; ++m)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) h[m][c] = hm[3 * m + c];
+  fixed_sub_blocks<0>(K, E, h, S, T);
+#pragma unroll
+  for (int s = 0; s < kSub; ++s)
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      if (sub_has(s, c)) h[sub_q(s) ^ (1 << c)][c] >>= min(T[c] - S[s], 63);
+#pragma unroll
+  for (int m = 0; m < 8; ++m)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) hm[3 * m + c] = h[m][c];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) Tm[c] = T[c];
+}
+
 // One element: lower and upper xy-modal layers -> the corner values of K0 u_e in
-// integers (lo: lower layer, hi: upper) and the factor that scales them.
+// integers (lo: lower layer, hi: upper), and the factor that scales them and
+// fixed_to_double's exponent per component.
 template <bool LOWER>
-__device__ __forceinline__ double element_fixed(const FixedK& K, const long long (&L)[4][3], int eL,
-                                                const long long (&U)[4][3], int eU, double f, long long (&lo)[4][3],
-                                                long long (&hi)[4][3]) {
-  const int E = max(eL, eU), dl = min(E - eL, 63), du = min(E - eU, 63);
+__device__ __forceinline__ void element_fixed(const FixedK& K, const long long (&L)[4][3], const int (&eL)[3],
+                                              const long long (&U)[4][3], const int (&eU)[3], double f,
+                                              long long (&lo)[4][3], long long (&hi)[4][3], double (&fs)[3],
+                                              int (&ex)[3]) {
+  int E[3], T[3], G[3];
   long long h[8][3];
 #pragma unroll
-  for (int m = 0; m < 4; ++m)
+  for (int c = 0; c < 3; ++c) {
+    E[c] = max(eL[c], eU[c]);
+    const int dl = min(E[c] - eL[c], 63), du = min(E[c] - eU[c], 63);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
+    for (int m = 0; m < 4; ++m) {
       const long long a = L[m][c] >> dl, b = U[m][c] >> du;
       h[m][c] = a + b;
       h[m + 4][c] = b - a;
     }
-  unsigned acc = 0;
+    h[0][c] = 0;  // a translation
+  }
+  // T: the largest mode of each component; G: of what enters each component's
+  // forces (by high words: T from above, G from below)
+  auto top = [&](int c, unsigned a) { return a ? E[c] - __clz((int)a) : kNoMode; };
 #pragma unroll
-  for (int m = 1; m < 8; ++m)
+  for (int c = 0; c < 3; ++c) G[c] = kNoMode;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
+  for (int c = 0; c < 3; ++c) {
+    unsigned s[8];
+#pragma unroll
+    for (int m = 1; m < 8; ++m) {
       const int t = (int)(h[m][c] >> 32);
-      acc |= (unsigned)(t ^ (t >> 31));
+      s[m] = (unsigned)(t ^ (t >> 31));
     }
-  const int n = min(__clz((int)acc), 31) - 3;  // |h| < 2^61 before and after: mode sums of 8 values below 2^58
-  int vh[8][3], vl[8][3];
-#pragma unroll
-  for (int m = 1; m < 8; ++m)
+    const int p = (c + 1) % 3, r = (c + 2) % 3, C = 1 << c, P = 1 << p, R = 1 << r;
+    const unsigned both = s[C] | s[7 ^ C], to_p = both | s[R | C] | s[P], to_r = both | s[P | C] | s[R];
+    const unsigned own = to_p | to_r | s[7];
+    T[c] = E[c] - __clz((int)own);
+    G[c] = max(G[c], top(c, own));
+    G[p] = max(G[p], top(c, to_p));
+    G[r] = max(G[r], top(c, to_r));
+  }
+  const int most = max(T[0], max(T[1], T[2])), least = min(G[0], min(G[1], G[2]));
+  // not for elements outside the grid (factor 0) and zero displacements
+  const bool general = most - least > kFixedGap && max(E[0], max(E[1], E[2])) > 1 &&
+                       ((unsigned)(__double2hiint(f) << 1) | (unsigned)__double2loint(f)) != 0u;
+  if (!__any_sync(0xffffffffu, general)) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const long long t = h[m][c] << n;
-      vl[m][c] = (int)t;
-      vh[m][c] = (int)(t >> 32) - (vl[m][c] >> 31);
+      const int k = E[c] - most - 3, kl = max(k, 0), kr = min(max(-k, 0), 63);
+#pragma unroll
+      for (int m = 1; m < 8; ++m) h[m][c] = (h[m][c] << kl) >> kr;
     }
-  long long w[8][3];
+    fs[0] = fs[1] = fs[2] = scale_exp(f, most - 1013 - K.exp, &ex[0]);
+    ex[1] = ex[2] = ex[0];
+    fixed_products<0>(K, h);
+  } else {
+    long long hm[24];
+    int Tm[3];
 #pragma unroll
-  for (int m = 0; m < 8; ++m)
+    for (int m = 0; m < 8; ++m)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const int q = m ^ (1 << c);
-      long long A = 0, M = 0;
+      for (int c = 0; c < 3; ++c) hm[3 * m + c] = h[m][c];
+    fixed_general(K, hm, E[0], E[1], E[2], Tm);
 #pragma unroll
-      for (int d = 0; d < 3; ++d)
-        if (modal_nz(q, c, d)) {
-          const int m2 = q ^ (1 << d);
-          A += (long long)vh[m2][d] * K.h[q][c][d];
-          M += (long long)vh[m2][d] * K.l[q][c][d];
-          M += (long long)vl[m2][d] * K.h[q][c][d];
-        }
-      w[m][c] = A + (M >> 32);
-    }
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) h[m][c] = hm[3 * m + c];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) T[c] = Tm[c];
+    // units 2^(T + 3 - 1080), coefficients 2^-exp, >> 64
+#pragma unroll
+    for (int c = 0; c < 3; ++c) fs[c] = scale_exp(f, T[c] - 1013 - K.exp, &ex[c]);
+  }
+  if (max(E[0], max(E[1], E[2])) == 0x7ff) fs[0] = fs[1] = fs[2] = __hiloint2double(0x7ff80000, 0);
   long long a[4][3];
   if (LOWER) {
 #pragma unroll
     for (int m = 0; m < 4; ++m)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) a[m][c] = w[m][c] - w[m + 4][c];
+      for (int c = 0; c < 3; ++c) a[m][c] = h[m][c] - h[m + 4][c];
     xy_inverse<long long>(a, lo);
   }
 #pragma unroll
   for (int m = 0; m < 4; ++m)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) a[m][c] = w[m][c] + w[m + 4][c];
+    for (int c = 0; c < 3; ++c) a[m][c] = h[m][c] + h[m + 4][c];
   xy_inverse<long long>(a, hi);
-  const double fs = scale_exp(f, E - 1016 - n - K.exp);  // units 2^(E - 1080), 2^-n, coefficients 2^-exp, >> 64
-  return E == 0x7ff ? __hiloint2double(0x7ff80000, 0) : fs;
 }
 
 // CTA height in warps.  FP32: 16 warps, one CTA per SM (127 registers); 8-warp
@@ -605,7 +733,7 @@ __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, in
   // FX: integer layers and their exponent, and a carry in corner values
   using M = typename std::conditional<FX, long long, T>::type;
   M Lm[4][3];
-  int eL = 0;
+  int eL[3] = {0, 0, 0};
   T carry[4][3], xown[3];
   T fprev;
   {
@@ -613,8 +741,8 @@ __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, in
     load_corners<T, IX, INTERIOR>(g, ca, x, k0 - 1, raw);
     drop_fixed(raw, load_bits(k0 - 1));
     M Lprev[4][3];
-    int ep = 0;
-    if constexpr (FX) ep = fixed_layer(raw, Lprev);
+    int ep[3];
+    if constexpr (FX) fixed_layer(raw, Lprev, ep);
     else xy_forward<T>(raw, Lprev);
     load_corners<T, IX, INTERIOR>(g, ca, x, k0, raw);
     drop_fixed(raw, load_bits(k0));
@@ -622,13 +750,15 @@ __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, in
     for (int c = 0; c < 3; ++c) xown[c] = raw[3][c];
     fprev = facload(k0 - 1);
     if constexpr (FX) {
-      eL = fixed_layer(raw, Lm);
+      fixed_layer(raw, Lm, eL);
       M none[4][3], up[4][3];
-      const T fs = element_fixed<false>(*fk, Lprev, ep, Lm, eL, fprev, none, up);
+      T fs[3];
+      int ex[3];
+      element_fixed<false>(*fk, Lprev, ep, Lm, eL, fprev, none, up, fs, ex);
 #pragma unroll
       for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) carry[cc][c] = fs * fixed_to_double(up[cc][c]);
+        for (int c = 0; c < 3; ++c) carry[cc][c] = fs[c] * fixed_to_double(up[cc][c], ex[c]);
     } else {
       xy_forward<T>(raw, Lm);
       T lo[4][3];
@@ -702,8 +832,8 @@ __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, in
 #pragma unroll
     for (int c = 0; c < 3; ++c) bk[c] = bnext[c], pk3[c] = pnext[c], xup[c] = nraw[3][c];
     M Um[4][3];
-    int eU = 0;
-    if constexpr (FX) eU = fixed_layer(nraw, Um);
+    int eU[3];
+    if constexpr (FX) fixed_layer(nraw, Um, eU);
     else if (EARLY) xy_forward<T>(nraw, Um);
     T raw[4][3];
     if (!EARLY && !FX) {
@@ -724,15 +854,18 @@ __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, in
     T cv[4][3];
     if constexpr (FX) {
       M lo[4][3], hi[4][3];
-      const T fs = element_fixed<true>(*fk, Lm, eL, Um, eU, f, lo, hi);
+      T fs[3];
+      int ex[3];
+      element_fixed<true>(*fk, Lm, eL, Um, eU, f, lo, hi, fs, ex);
 #pragma unroll
       for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          cv[cc][c] = fma(fs, fixed_to_double(lo[cc][c]), carry[cc][c]);
-          carry[cc][c] = fs * fixed_to_double(hi[cc][c]);
+          cv[cc][c] = fma(fs[c], fixed_to_double(lo[cc][c], ex[c]), carry[cc][c]);
+          carry[cc][c] = fs[c] * fixed_to_double(hi[cc][c], ex[c]);
         }
-      eL = eU;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) eL[c] = eU[c];
     } else {
       if (!EARLY) xy_forward<T>(raw, Um);
       T lo[4][3], hi[4][3];
