@@ -99,25 +99,27 @@ static EnergyK energy_blocks(const ModalK<double>& K) {
   return E;
 }
 
-// A warp owns 32 element columns in x and marches through kSensZ layers: the
+// A warp owns 32 element columns in x and marches through kz layers: the
 // xy-butterflies of a node layer serve the elements on both sides of it, and
 // the rigid translations (mode 0) are never formed.  About 100 FP64 instructions
 // an element, against 215 with the three transforms, the unsymmetric products
 // and pow per element; FP64 issue bound (81 % of
 // the pipe).  256x128x128: 825 us, 1851 before.
+// kz: at most kSensZ, fewer on grids whose chunks of 16 would leave SMs without
+// work, by the operator's chunk rule (starting an item costs a quarter of a layer).
 constexpr int kSensZ = 16;
 template <int N>
 __global__ void __launch_bounds__(128) sens_kernel(Grid g, const __grid_constant__ EnergyK K,
                                                    const double* __restrict__ rho, const double* __restrict__ u,
                                                    double Emin, double E0, double penal, double* __restrict__ dc,
-                                                   RedArgs red) {
-  const int nbx = (g.nx + 31) / 32, nby = (g.ny + 3) / 4, nzc = (g.nz + kSensZ - 1) / kSensZ;
+                                                   int kz, RedArgs red) {
+  const int nbx = (g.nx + 31) / 32, nby = (g.ny + 3) / 4, nzc = (g.nz + kz - 1) / kz;
   const long long items = (long long)nbx * nby * nzc;
   const double dE = E0 - Emin, scale = -penal * dE;
   double acc[1] = {0.0};
   for (long long item = blockIdx.x; item < items; item += gridDim.x) {
     const int i = (int)(item % nbx) * 32 + threadIdx.x, j = (int)(item / nbx % nby) * 4 + threadIdx.y;
-    const int k0 = (int)(item / nbx / nby) * kSensZ, k1 = min(k0 + kSensZ, g.nz);
+    const int k0 = (int)(item / nbx / nby) * kz, k1 = min(k0 + kz, g.nz);
     if (i >= g.nx || j >= g.ny) continue;
     const long long plane = 3LL * g.NX * g.NY;
     const double* col = u + 3 * ((long long)i + (long long)g.NX * j);
@@ -190,15 +192,17 @@ __global__ void __launch_bounds__(128) sens_kernel(Grid g, const __grid_constant
 }
 void launch_sensitivities(const Grid& g, const ModalK<double>& K, const double* rho, const double* u, double Emin,
                           double E0, double penal, double* dc, const RedArgs& red, cudaStream_t st) {
-  const long long items = (long long)((g.nx + 31) / 32) * ((g.ny + 3) / 4) * ((g.nz + kSensZ - 1) / kSensZ);
+  const long long tiles = (long long)((g.nx + 31) / 32) * ((g.ny + 3) / 4);
+  const int kz = std::min(kSensZ, op_chunk_layers(tiles, g.nz, 152, 0.25));
+  const long long items = tiles * ((g.nz + kz - 1) / kz);
   const int b = (int)std::min<long long>(items, 152 * 8);
   const EnergyK E = energy_blocks(K);
   switch (whole_penal(penal)) {
 #define HEXA_CASE(N) \
-  case N: sens_kernel<N><<<b, dim3(32, 4), 0, st>>>(g, E, rho, u, Emin, E0, penal, dc, red); break;
+  case N: sens_kernel<N><<<b, dim3(32, 4), 0, st>>>(g, E, rho, u, Emin, E0, penal, dc, kz, red); break;
     HEXA_CASE(1) HEXA_CASE(2) HEXA_CASE(3) HEXA_CASE(4) HEXA_CASE(5) HEXA_CASE(6)
 #undef HEXA_CASE
-    default: sens_kernel<-1><<<b, dim3(32, 4), 0, st>>>(g, E, rho, u, Emin, E0, penal, dc, red);
+    default: sens_kernel<-1><<<b, dim3(32, 4), 0, st>>>(g, E, rho, u, Emin, E0, penal, dc, kz, red);
   }
 }
 
