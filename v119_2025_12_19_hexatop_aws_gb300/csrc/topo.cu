@@ -105,8 +105,10 @@ static EnergyK energy_blocks(const ModalK<double>& K) {
 // an element, against 215 with the three transforms, the unsymmetric products
 // and pow per element; FP64 issue bound (81 % of
 // the pipe).  256x128x128: 825 us, 1851 before.
-// kz: at most kSensZ, fewer on grids whose chunks of 16 would leave SMs without
-// work, by the operator's chunk rule (starting an item costs a quarter of a layer).
+// kz: kSensZ where that gives every SM eight items (256x128x128: 846 us a call,
+// 856 in items of 6 layers), else fewer by the operator's chunk rule (starting
+// an item costs a quarter of a layer): 48x24x24 57 us in items of 8 layers, 35 in
+// items of two; 96x48x48 91 and 73 to 79 in items of 2 to 6.
 constexpr int kSensZ = 16;
 template <int N>
 __global__ void __launch_bounds__(128) sens_kernel(Grid g, const __grid_constant__ EnergyK K,
@@ -193,7 +195,8 @@ __global__ void __launch_bounds__(128) sens_kernel(Grid g, const __grid_constant
 void launch_sensitivities(const Grid& g, const ModalK<double>& K, const double* rho, const double* u, double Emin,
                           double E0, double penal, double* dc, const RedArgs& red, cudaStream_t st) {
   const long long tiles = (long long)((g.nx + 31) / 32) * ((g.ny + 3) / 4);
-  const int kz = std::min(kSensZ, op_chunk_layers(tiles, g.nz, 152, 0.25));
+  const bool many = tiles * ((g.nz + kSensZ - 1) / kSensZ) >= 152 * 8;
+  const int kz = many ? kSensZ : std::min(kSensZ, op_chunk_layers(tiles, g.nz, 152, 0.25));
   const long long items = tiles * ((g.nz + kz - 1) / kz);
   const int b = (int)std::min<long long>(items, 152 * 8);
   const EnergyK E = energy_blocks(K);
