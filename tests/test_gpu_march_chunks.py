@@ -31,3 +31,25 @@ def test_sensitivities_of_a_slab(ctx, rng, dims, penal):
         part, _ = sensitivities(_lib.make_grid(nx, ny, k1 - k0), rho[k0:k1].reshape(-1),
                                 np.ascontiguousarray(u[k0:k1 + 1]).reshape(-1), penal=penal, ctx=ctx)
         assert np.array_equal(part.reshape(k1 - k0, -1), dc[k0:k1])
+
+
+@pytest.mark.parametrize("dims", DIMS)
+def test_stresses_of_a_slab(ctx, rng, dims):
+    nx, ny, nz = dims
+    rho, u = fields(rng, dims)
+
+    def stress(k0, k1):
+        ne = nx * ny * (k1 - k0)
+        d = torch.from_numpy(rho[k0:k1].astype(np.float32)).cuda()
+        x = torch.from_numpy(u[k0:k1 + 1]).cuda()
+        out = [torch.empty(m * ne, device="cuda") for m in (3, 1, 6, 1, 3, 3)]
+        torch.cuda.synchronize()  # the context works on a stream of its own
+        grid = _lib.make_grid(nx, ny, k1 - k0)
+        ctx.check(ctx.lib.hexa_stress_field(ctx.h, C.byref(grid), _lib.ptr(x), _lib.ptr(d), 1.0, 0.3,
+                                            *[_lib.ptr(a) for a in out]))
+        return [a.cpu().numpy().reshape(k1 - k0, -1) for a in out]
+
+    whole = stress(0, nz)
+    for k0, k1 in [(0, 1), (nz - 3, nz), (5, 12)]:
+        for a, b in zip(whole, stress(k0, k1)):
+            assert np.array_equal(a[k0:k1], b)  # unit elements: the Jacobian is exact at any height

@@ -51,25 +51,29 @@ __device__ __forceinline__ void jacobi_rotate(float& spp, float& sqq, float& spq
   }
 }
 
-// A thread marches kStressZ elements of its column in z: the four nodes between
+// A thread marches kz elements of its column in z: the four nodes between
 // two elements are read and rounded once (conversions from FP64 run at the FP64
 // pipe's 2 per clock and SM), and the x and y parts of the Jacobian are formed
 // once.  Bound by instruction issue: the rotations' divisions and square roots,
 // then the index arithmetic, whose 64-bit divisions per element are gone.
 // 256x128x128 with the Voigt stress: 203 us (issue slots 74 % busy), 242 at one element per
 // thread; every operation on the values is the same, and so are the results.
+// kz: at most kStressZ, fewer where that would leave resident CTAs (7 an SM)
+// without work, by the operator's chunk rule; starting an item costs a fifth of a
+// layer.  A call on 48x24x24: 47 us in items of 8 layers, 22 in items of one;
+// 96x48x48: 50, 33 in items of two; 128x64x64: 57, 47 in items of four.
 constexpr int kStressZ = 8;
 template <typename TU>
 __global__ void __launch_bounds__(128) stress_kernel(Grid g, const TU* __restrict__ u, const float* __restrict__ density,
                                                      float E, float nu, float dx, float dy, float dz, int save_voigt,
-                                                     float* __restrict__ principal, float* __restrict__ vonmises,
+                                                     int kz, float* __restrict__ principal, float* __restrict__ vonmises,
                                                      float* __restrict__ voigt, float* __restrict__ l1,
                                                      float* __restrict__ dmax, float* __restrict__ dmin) {
-  const int nbx = (g.nx + 31) / 32, nby = (g.ny + 3) / 4, nzc = (g.nz + kStressZ - 1) / kStressZ;
+  const int nbx = (g.nx + 31) / 32, nby = (g.ny + 3) / 4, nzc = (g.nz + kz - 1) / kz;
   const long long items = (long long)nbx * nby * nzc;
   for (long long item = blockIdx.x; item < items; item += gridDim.x) {
     const int t = (int)(item / nbx), i = (int)(item - (long long)t * nbx) * 32 + threadIdx.x;
-    const int j = (t % nby) * 4 + threadIdx.y, k0 = t / nby * kStressZ, k1 = min(k0 + kStressZ, g.nz);
+    const int j = (t % nby) * 4 + threadIdx.y, k0 = t / nby * kz, k1 = min(k0 + kz, g.nz);
     if (i >= g.nx || j >= g.ny) continue;
     // node a of the element in the reference's order n1..n8 (Mesh.jl:45-53)
     constexpr int DI[8] = {0, 1, 1, 0, 0, 1, 1, 0}, DJ[8] = {0, 0, 1, 1, 0, 0, 1, 1}, DK[8] = {0, 0, 0, 0, 1, 1, 1, 1};
@@ -185,9 +189,11 @@ template <typename TU>
 void launch_stress(const Grid& g, const TU* u, const float* density, float E, float nu, float dx, float dy, float dz,
                    int save_voigt, float* principal, float* vonmises, float* voigt, float* l1, float* dmax,
                    float* dmin, cudaStream_t st) {
-  const long long items = (long long)((g.nx + 31) / 32) * ((g.ny + 3) / 4) * ((g.nz + kStressZ - 1) / kStressZ);
+  const long long tiles = (long long)((g.nx + 31) / 32) * ((g.ny + 3) / 4);
+  const int kz = std::min(kStressZ, op_chunk_layers(tiles, g.nz, 152 * 7, 0.2));
+  const long long items = tiles * ((g.nz + kz - 1) / kz);
   const int blocks = (int)std::min<long long>(items, 152LL * 64);
-  stress_kernel<TU><<<blocks, dim3(32, 4), 0, st>>>(g, u, density, E, nu, dx, dy, dz, save_voigt, principal, vonmises, voigt,
+  stress_kernel<TU><<<blocks, dim3(32, 4), 0, st>>>(g, u, density, E, nu, dx, dy, dz, save_voigt, kz, principal, vonmises, voigt,
                                             l1, dmax, dmin);
 }
 
