@@ -63,12 +63,13 @@ __device__ __forceinline__ void jacobi_rotate(float& spp, float& sqq, float& spq
 // layer.  A call on 48x24x24: 47 us in items of 8 layers, 22 in items of one;
 // 96x48x48: 50, 33 in items of two; 128x64x64: 57, 47 in items of four.
 constexpr int kStressZ = 8;
-template <typename TU>
+template <typename TU, int KZ>  // KZ 0: kz at run time
 __global__ void __launch_bounds__(128) stress_kernel(Grid g, const TU* __restrict__ u, const float* __restrict__ density,
                                                      float E, float nu, float dx, float dy, float dz, int save_voigt,
-                                                     int kz, float* __restrict__ principal, float* __restrict__ vonmises,
+                                                     int kz_, float* __restrict__ principal, float* __restrict__ vonmises,
                                                      float* __restrict__ voigt, float* __restrict__ l1,
                                                      float* __restrict__ dmax, float* __restrict__ dmin) {
+  const int kz = KZ ? KZ : kz_;
   const int nbx = (g.nx + 31) / 32, nby = (g.ny + 3) / 4, nzc = (g.nz + kz - 1) / kz;
   const long long items = (long long)nbx * nby * nzc;
   for (long long item = blockIdx.x; item < items; item += gridDim.x) {
@@ -193,8 +194,9 @@ void launch_stress(const Grid& g, const TU* u, const float* density, float E, fl
   const int kz = std::min(kStressZ, op_chunk_layers(tiles, g.nz, 152 * 7, 0.2));
   const long long items = tiles * ((g.nz + kz - 1) / kz);
   const int blocks = (int)std::min<long long>(items, 152LL * 64);
-  stress_kernel<TU><<<blocks, dim3(32, 4), 0, st>>>(g, u, density, E, nu, dx, dy, dz, save_voigt, kz, principal, vonmises, voigt,
-                                            l1, dmax, dmin);
+  const auto kernel = kz == kStressZ ? stress_kernel<TU, kStressZ> : stress_kernel<TU, 0>;
+  kernel<<<blocks, dim3(32, 4), 0, st>>>(g, u, density, E, nu, dx, dy, dz, save_voigt, kz, principal, vonmises, voigt, l1,
+                                         dmax, dmin);
 }
 
 template void launch_stress<double>(const Grid&, const double*, const float*, float, float, float, float, float, int,
