@@ -1094,7 +1094,7 @@ int hexa_oc_update(hexa_ctx* h, int64_t n, const double* x, const double* dc, co
   double* hi_d = c.vec<double>("o_hi", n);
   OcState* os = c.vec<OcState>("o_state", 1);
   const int nb = (int)std::min<long long>((n + 255) / 256, 152 * 4);
-  if (!xd || !cd || !vd || !od || !lam_d || !t || !lo_d || !hi_d || !os || !c.ensure_partials((size_t)nb * 33 + 64))
+  if (!xd || !cd || !vd || !od || !lam_d || !t || !lo_d || !hi_d || !os || !c.ensure_partials((size_t)nb * 32 + 64))
     return HEXA_ERR_NOMEM;
   // The multiplier is that of the 88-line code's bisection on lambda in
   // [0, 1e9], carried to (l2 - l1)/(l1 + l2) <= 1e-12 where that stops at

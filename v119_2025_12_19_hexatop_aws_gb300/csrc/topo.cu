@@ -305,9 +305,9 @@ __global__ void __launch_bounds__(256) oc_prepare_kernel(const double* __restric
                                                          double* __restrict__ lo, double* __restrict__ hi,
                                                          double* __restrict__ part, OcState* __restrict__ st) {
   const float s0 = 3.1622776e-5f;  // 1 / sqrt(1e9)
-  float acc[kOcCand + 1];  // and the volume of the lower limits
+  float acc[kOcCand];
 #pragma unroll
-  for (int q = 0; q <= kOcCand; ++q) acc[q] = 0.f;
+  for (int q = 0; q < kOcCand; ++q) acc[q] = 0.f;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
     const OcElem el = oc_elem(x[e], dc[e], dv[e], move);
     t[e] = el.t;
@@ -320,18 +320,22 @@ __global__ void __launch_bounds__(256) oc_prepare_kernel(const double* __restric
       acc[q] += fmaxf(l, fminf(h, be));  // NaN: h
       be += be;
     }
-    acc[kOcCand] += l;
   }
-  __shared__ double tot[kOcCand + 1];
-  if (!oc_block_totals<kOcCand + 1, float>(acc, part, &st->ticket, tot) || threadIdx.x != 0) return;
+  __shared__ double tot[kOcCand];
+  if (!oc_block_totals<kOcCand, float>(acc, part, &st->ticket, tot) || threadIdx.x != 0) return;
   int k = 0;
   while (k < kOcCand && !(tot[k] > target)) ++k;
   const double s00 = 1.0 / sqrt(1e9);
   auto at = [&](int q) { return q < 0 ? 0.0 : s00 * exp2((double)q); };
   st->state = 0;
-  // no multiplier of the range reaches the target, or the lower limits exceed it
-  // (by more than FP32 sums are off; 48 steps would look for the root in vain), or NaN
-  if (k == kOcCand || tot[kOcCand] > 1.001 * target) {
+  // the volume at the upper multiplier exceeds the target, by more than FP32 sums
+  // are off: so it does at every multiplier of the bisection, which ends there
+  if (tot[0] > 1.001 * target) {
+    st->root = 1e-150;
+    st->state = 1;
+    return;
+  }
+  if (k == kOcCand) {  // no multiplier of the range reaches the target (or NaN)
     st->state = 2;
     return;
   }
