@@ -104,7 +104,7 @@ __device__ __forceinline__ double scale2(double v, int faces) {
 // neighbouring tiles read p_old).  The preconditioner is D^-1 times the inner
 // nodes' diagonal, z = 2^faces r: a constant factor in z cancels in the
 // iterates, and the common case needs no product.  On 256x128x128 in FP64 it
-// takes 0.169 ms (FP64 pipe 76 % busy, 18 FP64 instructions a node) where the
+// takes 0.169 ms (FP64 pipe 81 % busy, 18 FP64 instructions a node) where the
 // element-wise product and the p pass took 0.539 + 0.016 ms; with the update
 // below the whole filter (10 iterations) went from 6.83 to 2.44 ms.
 //

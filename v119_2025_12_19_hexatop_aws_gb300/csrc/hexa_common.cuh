@@ -251,7 +251,7 @@ __device__ __forceinline__ void finalize_scalars(const RedArgs& r, const double*
 // lanes at 256 threads instead of 8 x 5 + 5: an FP64 instruction holds its
 // scheduler for 64 cycles), and the warps that sum are spread over an SM's
 // schedulers by the blocks' number.  95x47x61 filter call 628 -> 604 us,
-// 256x128x128 filter 2448 -> 2427, batches 339 -> 335 us an iteration.
+// 256x128x128 filter 2448 -> 2427.
 template <int NSUM, int NTHR = 0>
 __device__ __forceinline__ void block_reduce_finalize_at(const RedArgs& r, double (&v)[NSUM], int col, long long bid,
                                                          long long nb, long long base, long long step) {

@@ -52,7 +52,7 @@ using namespace hexa;
 
 constexpr long long kMaxNodes = HEXA_NOALLOC_MAX_NODES;
 constexpr int kVecs = 5;                // x, r, p (two, alternating), q
-constexpr long long kHeader = 4224;      // doubles: scalars, ticket, results, partials
+constexpr long long kHeader = 4224;      // doubles: scalars, ticket, partials
 constexpr long long kScratchDoubles = kHeader + kVecs * kMaxNodes;
 constexpr int kMaxDevices = 64;
 
@@ -151,7 +151,6 @@ extern "C" int hexa_filter_noalloc(const hexa_grid* g, const double* rho_in, dou
 
   PcgScalars* s = (PcgScalars*)base;
   unsigned* ticket = (unsigned*)(base + 64);
-  double* result = base + 96;
   double* partials = base + 128;
   const long long nn = G.nnode();
   double* vec = base + kHeader;

@@ -784,7 +784,7 @@ __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, in
   // x, b and the previous iterate two layers past the register prefetch, into
   // L2: 384x192x192 Chebyshev step 0.2207 -> 0.2160 ms, residual 0.2086 ->
   // 0.2032, apply with p.Ap 0.2022 -> 0.1978; three to six layers gain less.
-  // Only in the kernels of grids whose vectors overflow L2 (see launch_op).
+  // Only in the kernels of grids of which three vectors overflow L2 (see launch_op).
   const IX touch0 = (IX)3 * ((IX)min(in, g.NX - 1) + (IX)g.NX * min(jn, g.NY - 1));
   auto touch_l2 = [&](int k) {
     if (!TOUCH || k + 3 >= k1) return;

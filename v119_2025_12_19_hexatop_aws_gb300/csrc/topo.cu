@@ -103,7 +103,7 @@ static EnergyK energy_blocks(const ModalK<double>& K) {
 // xy-butterflies of a node layer serve the elements on both sides of it, and
 // the rigid translations (mode 0) are never formed.  About 100 FP64 instructions
 // an element, against 215 with the three transforms, the unsymmetric products
-// and pow per element; FP64 issue bound (81 % of
+// and pow per element; FP64 issue bound (85 % of
 // the pipe).  256x128x128: 825 us, 1851 before.
 // kz: kSensZ where that gives every SM eight items (256x128x128: 846 us a call,
 // 856 in items of 6 layers), else fewer by the operator's chunk rule (starting
