@@ -1593,9 +1593,6 @@ void launch_op(int mode, const OpArgs<T>& a0, cudaStream_t st) {
   constexpr int TYW = op_tyw<T>();
   OpArgs<T> a = a0;
   op_tiles<T>(a.g, a.kchunk, &a.tiles_x, &a.tiles_y, &a.nchunks);
-  const long long items = (long long)a.tiles_x * a.tiles_y * a.nchunks;
-  const int grid = (int)std::min<long long>(items, resident_ctas<T>(mode));
-  const dim3 block(32, TYW);
   const bool i32 = a.g.ndof() < (1LL << 30) && a.g.nelem() < (1LL << 30);
   if constexpr (sizeof(T) == 4) {
     if (a.ncol <= 1 && op_form() == 1) {
@@ -1608,7 +1605,14 @@ void launch_op(int mode, const OpArgs<T>& a0, cudaStream_t st) {
       const FixedK fk = fixed_blocks(a.K);
       if (fk.ok && launch_op_fixed(mode, a, fk, st)) return;
     }
+    if (mode != OP_RESID_NORM) {  // chunks were picked for the integer form's taller tiles
+      a.kchunk = op_pick_kchunk<T>(a.g, OP_RESID_NORM);
+      op_tiles<T>(a.g, a.kchunk, &a.tiles_x, &a.tiles_y, &a.nchunks);
+    }
   }
+  const long long items = (long long)a.tiles_x * a.tiles_y * a.nchunks;
+  const int grid = (int)std::min<long long>(items, resident_ctas<T>(mode));
+  const dim3 block(32, TYW);
   if (a.ncol > 1) {  // multi-column forms (no reductions): apply, residual and the two smoothing steps
     if (mode == OP_APPLY) {
       if (i32) op_kernel<T, OP_APPLY, TYW, int, true><<<grid, block, 0, st>>>(a);
