@@ -804,8 +804,7 @@ __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, in
   // kSumLayers layers (96 terms), accS over those (an item may be 400 layers
   // long); both go to the FP64 accumulator at the end.  FP64 arithmetic in the
   // march would run at GB300's FP64 rate: folding into FP64 every 32 layers took
-  // 203.3 us for the 384x192x192 product with its dot and 239.8 for the residual
-  // norm.
+  // 203.3 us for the 384x192x192 product with its dot, this 196.7.
   constexpr bool SUMS = sizeof(T) == 4 && (MODE == OP_APPLY_DOT || BM == OP_RESID_NORM || DOTB);
   constexpr int kSumLayers = 32;
   T accT = T(0), accS = T(0);
@@ -819,8 +818,9 @@ __device__ __forceinline__ void op_item(const A& a, const FixedK* fk, int tx, in
 
   // three layers per unrolled step for the Chebyshev forms, two for the rest
   // (on the 384x192x192 grid: Chebyshev step 0.2191 ms at 3 against 0.2248
-  // at 2 and 0.2475 at 1; Jacobi step 0.2006 at 3, 0.1983 at 2)
-#pragma unroll(FX ? 1 : (BM == OP_CHEB2 ? 3 : 2))
+  // at 2 and 0.2475 at 1; Jacobi step 0.2006 at 3, 0.1983 at 2); not unrolled
+  // for the FP32 residual norm (0.2192 against 0.2428, which spills)
+#pragma unroll((FX || (sizeof(T) == 4 && BM == OP_RESID_NORM)) ? 1 : (BM == OP_CHEB2 ? 3 : 2))
   for (int k = k0; k < k1; ++k) {
     if (!PRE) {
       load_corners<T, IX, INTERIOR>(g, ca, x, k + 1, nraw);
