@@ -301,17 +301,18 @@ __device__ __forceinline__ void element_modal<float>(const ModalK<float>& K, con
 //   * the strain modes are normalised by their largest (60 bits), so the
 //     precision follows the strains, not the rigid motion they were taken from;
 //   * the modal blocks multiply as two 32-bit halves (vh ch, vh cl, vl ch
-//     accumulated in 64 bits and rounded; the dropped vl cl is below 2^-58 of the
-//     largest mode times the largest coefficient), the inverse butterflies are
-//     exact.
+//     accumulated in 64 bits and rounded; up to three vl cl dropped): off by at
+//     most 2^-55 of the largest mode times the largest coefficient, by about 2^-58
+//     on average; the inverse butterflies are exact.
 // The modes that enter one component's forces can be far smaller than others
 // that do not (a force in x feels four of the seven modes of u_z).  Where
-// they are within 2^-3 of the largest, for each component, one
-// scale serves the element; elsewhere (kFixedGap) each of the eleven sub-blocks
-// that couple has its own, and each component's sums are aligned to the largest term
-// that they have.  So a rounding is below about 2^-55 of the largest term of the
-// force component that it enters, where FP64 rounds at 2^-53 of every
-// intermediate sum.
+// they are within 2^-3 of the largest, for each component, one scale serves the
+// element; elsewhere (kFixedGap) each of the eleven sub-blocks that couple has
+// its own, and each component's sums are aligned to the largest term that they
+// have.  So a mode's error is at most 2^-52 of the largest term of the force
+// component that it enters and about 2^-56 on average, where FP64 rounds at
+// 2^-53 of every intermediate sum; weak coefficients (to 2^-6 of the largest)
+// raise both by their ratio, where nothing stronger enters with them.
 // Chosen when the smallest modal coefficient is within 2^-6 of the largest
 // (bricks and nu in ordinary use; not nu = 0, nu near 0.5 or needle elements),
 // else the FP64 form.  The norm of the true residual (OP_RESID_NORM), which a
