@@ -77,3 +77,13 @@ def test_subnormal_displacements(ctx, oracle, rng):
     y, _ = product(ctx, oracle, fac, u * 2.0 ** -1074)
     # sums of up to 8 elements, each rounded to the spacing 2^-1074
     assert np.abs(y * 2.0 ** 1000 * 2.0 ** 74 - ref).max() <= 8.0
+
+
+@pytest.mark.parametrize("contrast", [False, True])
+@pytest.mark.parametrize("eps", [1e-3, 1e-8, 1e-10, 1e-13])
+def test_small_strains_on_a_large_translation(ctx, oracle, rng, contrast, eps):
+    fac = factors(rng, contrast)
+    u = noise(rng, eps, eps, eps) - 1.7
+    _, ref = product(ctx, oracle, fac, u + 1.7)  # exact: values within a factor of two of 1.7
+    y, _ = product(ctx, oracle, fac, u)
+    assert np.abs(y - ref).max() <= 1e-13 * np.abs(ref).max()
